@@ -100,8 +100,8 @@ class CudaWork : public AsyncWork {
         const std::string m = status_message(*comm_);
         if (!m.empty()) throw_dist_error(m);
       }
-    } else if (!same_stream_) {
-      C10_CUDA_CHECK(cudaStreamWaitEvent(c10::cuda::getCurrentCUDAStream(device_.index()).stream(), end_->ev, 0));
+    } else {
+      synchronize();
     }
     std::exception_ptr e;
     {
@@ -113,7 +113,12 @@ class CudaWork : public AsyncWork {
   }
 
   void synchronize() override {
-    if (!same_stream_ && end_) C10_CUDA_CHECK(cudaStreamWaitEvent(c10::cuda::getCurrentCUDAStream(device_.index()).stream(), end_->ev, 0));
+    if (same_stream_ || !end_) return;
+    const cudaStream_t cur = c10::cuda::getCurrentCUDAStream(device_.index()).stream();
+    if (!stream_ || stream_->stream() != cur) C10_CUDA_CHECK(cudaStreamWaitEvent(cur, end_->ev, 0));
+    // From here on the issuing stream runs after the kernels, so the tensors may be freed in its order. (Waiting on
+    // another stream says nothing about the one they were allocated for: the watchdog keeps them then.)
+    if (keep_ && cur == issued_from_) keep_->drop();
   }
 
   int cudaDevice() const override { return device_.index(); }
@@ -140,6 +145,8 @@ class CudaWork : public AsyncWork {
   std::shared_ptr<PooledEvent> start_, end_;
   std::optional<c10::cuda::CUDAStream> stream_;
   std::shared_ptr<CudaComm> comm_;
+  std::shared_ptr<Watchdog::KeepAlive> keep_;
+  cudaStream_t issued_from_ = nullptr;
   bool blocking_ = false, same_stream_ = false, host_blocking_ = false, timed_ = false;
   std::chrono::milliseconds timeout_{10000};
   at::Device device_;
@@ -158,16 +165,24 @@ Watchdog& Watchdog::get() {
 Watchdog::Watchdog() : th_([this] { loop(); }) {}
 
 void Watchdog::enqueue(Item item) {
+  bool wake;
   {
     std::lock_guard<std::mutex> g(mu_);
     q_.push_back(std::move(item));
+    wake = asleep_;
+    asleep_ = false;
   }
-  cv_.notify_all();
+  // A busy program issues a collective every few microseconds: while the thread is on its millisecond beat there is
+  // no need to wake it (a futex call here, and two threads in the driver at once). Waiters use the events directly.
+  if (wake) cv_.notify_all();
 }
 
 void Watchdog::drain() {
   std::unique_lock<std::mutex> l(mu_);
+  ++drainers_;
+  cv_.notify_all();
   cv_.wait(l, [this] { return q_.empty() && !busy_; });
+  --drainers_;
 }
 
 void Watchdog::stop() {
@@ -179,68 +194,99 @@ void Watchdog::stop() {
   if (th_.joinable()) th_.join();
 }
 
+void Watchdog::complete(Item& it, bool gave_up) {
+  try {
+    Telemetry::get().record_complete(it.flight_slot, it.seq);
+    std::string m = it.comm && !gave_up ? status_message(*it.comm) : std::string();
+    auto work = it.work.lock();
+    if (gave_up) {
+      static std::vector<std::shared_ptr<KeepAlive>>* leaked = new std::vector<std::shared_ptr<KeepAlive>>();
+      leaked->push_back(std::move(it.keep));
+      m = "ccl: watchdog gave up on work " + std::to_string(it.seq) + " after its timeout of " + std::to_string(it.timeout.count()) +
+          " ms (the kernel did not end after the abort)";
+    } else if (!m.empty()) {
+      std::cerr << "[ccl] " << m << "\n" << Telemetry::get().dump_flight();
+    }
+    if (it.keep) it.keep->drop();
+    if (!work) return;  // nobody holds it any more
+    if (m.empty()) work->finishOk();
+    else work->finishError(std::make_exception_ptr(c10::DistBackendError(c10::SourceLocation{"ccl", __FILE__, __LINE__}, m)));
+  } catch (...) {
+    if (auto work = it.work.lock()) work->finishError(std::current_exception());
+  }
+}
+
+// Every device wait of the library is bounded (spin budget <= the group's timeout), so a work normally ends or fails by
+// itself. The deadline is the backstop for a spin budget configured longer than the timeout: kGrace after the timeout the
+// watchdog raises the communicator's abort word (every bounded wait samples it and returns within about a millisecond,
+// status "aborted"); if the event has not fired kGiveUp later either, the work is failed without it and its tensors are
+// leaked rather than freed under a kernel that may still run.
+bool Watchdog::retire(std::deque<Item>& q) {
+  constexpr auto kGrace = std::chrono::seconds(2), kGiveUp = std::chrono::seconds(10);
+  while (!q.empty()) {
+    // Works of one stream complete in order: one query at the end of a run of them answers for the whole run.
+    size_t n = 1;
+    while (n < q.size() && q[n].stream == q[0].stream && q[0].stream) ++n;
+    while (n > 1 && !q[n - 1].end->query()) n /= 2;
+    if (n == 1 && !q[0].end->query()) {
+      Item& it = q[0];
+      const auto now = std::chrono::steady_clock::now();
+      if (it.since == std::chrono::steady_clock::time_point{}) it.since = now;
+      if (it.timeout.count() <= 0) return false;
+      const auto waited = now - it.since;
+      if (!it.raised && waited > it.timeout + kGrace) {
+        it.raised = true;
+        std::cerr << "[ccl] watchdog: work " << it.seq << " is past its timeout of " << it.timeout.count()
+                  << " ms; aborting the communicator\n" << Telemetry::get().dump_flight();
+        if (it.comm) it.comm->abort();
+      }
+      if (!it.raised || waited <= it.timeout + kGrace + kGiveUp) return false;
+      complete(it, true);
+      q.pop_front();
+      continue;
+    }
+    for (; n > 0; --n) {
+      complete(q[0], false);
+      q.pop_front();
+    }
+  }
+  return true;
+}
+
 void Watchdog::loop() {
+  std::deque<Item> mine;  // taken out of q_, in issue order
+  int idle = 0;
   std::unique_lock<std::mutex> l(mu_);
   while (true) {
-    cv_.wait(l, [this] { return stop_ || !q_.empty(); });
-    if (stop_ && q_.empty()) return;
-    Item it = std::move(q_.front());
-    q_.pop_front();
+    if (q_.empty() && mine.empty()) {
+      if (stop_) return;
+      // a program that has issued nothing for a while: sleep until it does
+      if (++idle > 50) {
+        asleep_ = true;
+        cv_.wait(l, [this] { return stop_ || !q_.empty(); });
+        asleep_ = false;
+        idle = 0;
+      } else {
+        cv_.wait_for(l, std::chrono::milliseconds(1));
+      }
+      continue;
+    }
+    idle = 0;
+    while (!q_.empty()) {
+      mine.push_back(std::move(q_.front()));
+      q_.pop_front();
+    }
     busy_ = true;
     l.unlock();
-    try {
-      // works complete in stream order, so waiting on the oldest one first is enough
-      // a coarse poll: waiters use the event directly, the watchdog only retires work.
-      // Deadline: every device wait of the library is bounded (spin budget <= the group's timeout), so a work
-      // normally ends or fails by itself. The deadline is the backstop for a spin budget configured longer than
-      // the timeout: kGrace after the timeout the watchdog raises the communicator's abort word (every bounded
-      // wait samples it and returns within about a millisecond, status "aborted"); if the event has not fired
-      // kGiveUp later either, the work is failed without it and its tensors are leaked rather than freed under
-      // a kernel that may still run.
-      constexpr auto kGrace = std::chrono::seconds(2), kGiveUp = std::chrono::seconds(10);
-      const auto t0 = std::chrono::steady_clock::now();
-      bool raised = false, gave_up = false;
-      while (!it.end->query()) {
-        if (it.timeout.count() > 0) {
-          const auto waited = std::chrono::steady_clock::now() - t0;
-          if (!raised && waited > it.timeout + kGrace) {
-            raised = true;
-            std::cerr << "[ccl] watchdog: work " << it.seq << " is past its timeout of " << it.timeout.count()
-                      << " ms; aborting the communicator\n" << Telemetry::get().dump_flight();
-            if (it.comm) it.comm->abort();
-          }
-          if (raised && waited > it.timeout + kGrace + kGiveUp) {
-            gave_up = true;
-            break;
-          }
-        }
-        std::this_thread::sleep_for(std::chrono::microseconds(200));
-      }
-      Telemetry::get().record_complete(it.work->flight_slot, it.seq);
-      if (gave_up) {
-        static std::vector<std::vector<at::Tensor>>* leaked = new std::vector<std::vector<at::Tensor>>();
-        leaked->push_back(std::move(it.keep));
-        it.work->finishError(std::make_exception_ptr(c10::DistBackendError(
-            c10::SourceLocation{"ccl", __FILE__, __LINE__},
-            "ccl: watchdog gave up on work " + std::to_string(it.seq) + " after its timeout of " +
-                std::to_string(it.timeout.count()) + " ms (the kernel did not end after the abort)")));
-      } else {
-        std::string m = it.comm ? status_message(*it.comm) : std::string();
-        if (m.empty()) {
-          it.work->finishOk();
-        } else {
-          std::cerr << "[ccl] " << m << "\n" << Telemetry::get().dump_flight();
-          it.work->finishError(std::make_exception_ptr(
-              c10::DistBackendError(c10::SourceLocation{"ccl", __FILE__, __LINE__}, m)));
-        }
-      }
-    } catch (...) {
-      it.work->finishError(std::current_exception());
-    }
-    it = Item{};
+    const bool all = retire(mine);
     l.lock();
-    busy_ = false;
-    cv_.notify_all();
+    busy_ = !mine.empty();
+    if (all) {
+      cv_.notify_all();
+      if (q_.empty()) continue;
+    }
+    // a coarse beat, finer while somebody waits for the queue to empty
+    cv_.wait_for(l, drainers_ ? std::chrono::microseconds(100) : std::chrono::microseconds(1000));
   }
 }
 
@@ -424,7 +470,7 @@ c10::cuda::CUDAStream CudaBackendImpl::comm_stream(const at::Device& device) {
 c10::intrusive_ptr<c10d::Work> CudaBackendImpl::run(c10d::OpType type, const char* title, const at::Device& device,
                                                     const LaunchFn& fn, const std::vector<at::Tensor>& keep,
                                                     std::vector<at::Tensor> outs, std::vector<std::vector<at::Tensor>> nested,
-                                                    bool use_nested, uint64_t bytes, bool host_blocking) {
+                                                    bool use_nested, uint64_t bytes, bool async_op, bool host_blocking) {
   CudaComm& c = comm(device);
   if (c.poll_status() != 0) throw_dist_error(status_message(c));
   const int dev = c.device();
@@ -442,9 +488,11 @@ c10::intrusive_ptr<c10d::Work> CudaBackendImpl::run(c10d::OpType type, const cha
   work->timed_ = pg_->timingEnabled();
 
   c10::cuda::CUDAStream cur = c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)dev);
-  c10::cuda::CUDAStream stream = same ? cur : comm_stream(device);
+  const bool fork = async_op && !same;
+  c10::cuda::CUDAStream stream = fork ? comm_stream(device) : cur;
   work->stream_ = stream;
-  if (!same) {
+  work->issued_from_ = cur.stream();
+  if (fork) {
     // fork: the communication stream waits for what the caller has enqueued so far. One event
     // per backend is enough: a wait captures the record that precedes it.
     if (!fork_event_) fork_event_ = acquire_event(dev, false);
@@ -470,10 +518,17 @@ c10::intrusive_ptr<c10d::Work> CudaBackendImpl::run(c10d::OpType type, const cha
   work->flight_slot = Telemetry::get().record_start(seq, title, "cuda", bytes, algo.c_str());
 
   Watchdog::Item item;
-  item.work = work;
+  item.work = c10::weak_intrusive_ptr<AsyncWork>(work);
   item.end = work->end_;
   item.comm = comm_;
-  item.keep = keep;  // keeps the tensors alive until the kernels have run (instead of record_stream)
+  if (fork) {
+    // keeps the tensors alive while another stream uses them (instead of record_stream)
+    item.keep = std::make_shared<Watchdog::KeepAlive>();
+    item.keep->tensors = keep;
+    work->keep_ = item.keep;
+  }
+  item.stream = stream.stream();
+  item.flight_slot = work->flight_slot;
   item.seq = seq;
   item.timeout = pg_->timeout();
   Watchdog::get().enqueue(std::move(item));
@@ -548,9 +603,11 @@ c10::intrusive_ptr<c10d::Work> CudaBackendImpl::p2p(bool is_send, at::Tensor& te
   w->end_ = acquire_event(dev, false);
   C10_CUDA_CHECK(cudaEventRecord(w->end_->ev, stream.stream()));
   Watchdog::Item item;
-  item.work = w;
+  item.work = c10::weak_intrusive_ptr<AsyncWork>(w);
   item.end = w->end_;
-  item.keep = {tensor};
+  item.keep = std::make_shared<Watchdog::KeepAlive>();
+  item.keep->tensors = {tensor};
+  item.stream = stream.stream();
   item.seq = seq;
   item.timeout = pg_->timeout();
   Watchdog::get().enqueue(std::move(item));
@@ -577,10 +634,12 @@ c10::intrusive_ptr<c10d::Work> CudaBackendImpl::p2p_group_end() {
   w->end_ = acquire_event(dev, false);
   C10_CUDA_CHECK(cudaEventRecord(w->end_->ev, stream.stream()));
   Watchdog::Item item;
-  item.work = w;
+  item.work = c10::weak_intrusive_ptr<AsyncWork>(w);
   item.end = w->end_;
-  item.keep = std::move(p2p_batch_tensors_);
+  item.keep = std::make_shared<Watchdog::KeepAlive>();
+  item.keep->tensors = std::move(p2p_batch_tensors_);
   p2p_batch_tensors_.clear();
+  item.stream = stream.stream();
   item.seq = seq;
   item.timeout = pg_->timeout();
   Watchdog::get().enqueue(std::move(item));

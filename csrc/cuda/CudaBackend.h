@@ -38,12 +38,15 @@ class CudaBackendImpl {
   using LaunchFn = std::function<std::string(CudaComm&, cudaStream_t)>;  // returns the algorithm tag
 
   // Runs `fn` on the communication stream (or the current stream in same-stream mode) with the
-  // proper event dependencies and returns the Work. `keep` tensors are kept alive / recorded on
-  // the stream. `host_blocking`: wait() blocks the host until completion (barrier).
+  // proper event dependencies and returns the Work. `keep` tensors are kept alive until the caller
+  // has waited for the work on the stream it was issued from, or the kernels have run.
+  // `host_blocking`: wait() blocks the host until completion (barrier). `async_op` false: the caller
+  // waits before it does anything else (`async_op=False` in torch.distributed), so the kernels go
+  // straight onto its stream: no fork, no join, and the tensors need no keeping.
   c10::intrusive_ptr<c10d::Work> run(c10d::OpType type, const char* title, const at::Device& device,
                                      const LaunchFn& fn, const std::vector<at::Tensor>& keep,
                                      std::vector<at::Tensor> outs, std::vector<std::vector<at::Tensor>> nested,
-                                     bool use_nested, uint64_t bytes, bool host_blocking = false);
+                                     bool use_nested, uint64_t bytes, bool async_op = true, bool host_blocking = false);
 
   // NCCL p2p (send / recv, batched between start/endCoalescing).
   c10::intrusive_ptr<c10d::Work> p2p(bool is_send, at::Tensor& tensor, int peer, bool batched);
@@ -80,16 +83,34 @@ class CudaBackendImpl {
 
 // The process-wide watchdog: keeps in-flight CUDA work alive until its end event fires, then
 // finishes it (or fails it when the communicator reported a device-side timeout).
+//
+// It holds the Work weakly and the tensors through a KeepAlive that wait() may empty first: a program
+// that enqueues faster than the GPU runs would otherwise find every temporary of every collective
+// still owned by this thread, and the allocator growing until it has to synchronise and free.
 class Watchdog {
  public:
   static Watchdog& get();
+  struct KeepAlive {
+    std::mutex mu;
+    std::vector<at::Tensor> tensors;
+    void drop() {
+      std::vector<at::Tensor> gone;  // freed outside the lock
+      std::lock_guard<std::mutex> g(mu);
+      gone.swap(tensors);
+    }
+  };
   struct Item {
-    c10::intrusive_ptr<c10d::ProcessGroupCCL::AsyncWorkCCL> work;
+    c10::weak_intrusive_ptr<c10d::ProcessGroupCCL::AsyncWorkCCL> work;
     std::shared_ptr<PooledEvent> end;
     std::shared_ptr<CudaComm> comm;
-    std::vector<at::Tensor> keep;
-    uint64_t seq;
-    std::chrono::milliseconds timeout{0};  // the group's timeout; 0 = no deadline (see Watchdog::loop)
+    std::shared_ptr<KeepAlive> keep;       // null: nothing to keep
+    cudaStream_t stream = nullptr;         // works of one stream complete in the order they were issued
+    size_t flight_slot = 0;
+    uint64_t seq = 0;
+    std::chrono::milliseconds timeout{0};  // the group's timeout; 0 = no deadline (see Watchdog::retire)
+    std::chrono::steady_clock::time_point since{};  // when this item came to the head of the queue
+    bool raised = false;                   // the communicator has been told to abort
+    Item() : work(c10::intrusive_ptr<c10d::ProcessGroupCCL::AsyncWorkCCL>()) {}
   };
   void enqueue(Item item);
   void drain();  // blocks until every queued work has completed
@@ -98,11 +119,15 @@ class Watchdog {
  private:
   Watchdog();
   void loop();
+  static bool retire(std::deque<Item>& q);  // completes what has run; false if the head is still pending
+  static void complete(Item& it, bool gave_up);
   std::mutex mu_;
   std::condition_variable cv_;
   std::deque<Item> q_;
   bool stop_ = false;
-  bool busy_ = false;
+  bool busy_ = false;      // items taken out of q_ are not all retired yet
+  bool asleep_ = false;    // the thread waits without a time limit: only then has enqueue() to wake it
+  int drainers_ = 0;       // threads in drain()
   std::thread th_;
 };
 

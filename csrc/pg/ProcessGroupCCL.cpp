@@ -552,6 +552,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::broadcast(std::vector<at::Tensor>& ten
   ccl::check_single_tensor(tensors);
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::broadcast", to_ivalues(tensors));
   CCL_OP_PROLOGUE("broadcast", tensors[0], flow_str((int)opts.rootRank, rank_), tensors_str(tensors), nbytes(tensors))
+  const bool async_op = issuedAsync(opts.asyncOp);
   at::Tensor t = tensors[0];
   const int root = (int)opts.rootRank;
   const auto tmo = opTimeout(opts.timeout);
@@ -567,7 +568,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::broadcast(std::vector<at::Tensor>& ten
           a.mode = ccl::kBroadcast;
           C10_CUDA_CHECK(c.rooted({a}, s));
           return std::string("rooted");
-        }, {t}, {t}, {}, false, bytes__);
+        }, {t}, {t}, {}, false, bytes__, async_op);
   } else {
     w = enqueueCpu(OpType::BROADCAST, "oneccl_bindings_for_pytorch::cpu::broadcast",
         [t, root, tmo](ccl::cpu::ShmComm& c) {
@@ -583,7 +584,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::broadcast(std::vector<at::Tensor>& ten
 // ------------------------------------------------------------------------------------------
 static c10::intrusive_ptr<Work> allreduce_impl(ProcessGroupCCL& pg, std::vector<at::Tensor> ts, const ReduceOp& rop,
                                                std::chrono::milliseconds tmo, OpType type, bool on_cuda,
-                                               uint64_t seq, size_t flight, uint64_t bytes,
+                                               uint64_t seq, size_t flight, uint64_t bytes, bool async_op,
                                                const std::function<c10::intrusive_ptr<Work>(std::function<void(ccl::cpu::ShmComm&)>, std::vector<at::Tensor>)>& cpu_enqueue) {
   const int W = pg.getSize();
   if (on_cuda) {
@@ -634,7 +635,7 @@ static c10::intrusive_ptr<Work> allreduce_impl(ProcessGroupCCL& pg, std::vector<
             tag = ch.algo == ccl::Algo::kOneShot ? "oneshot" : (ch.algo == ccl::Algo::kNvls ? "nvls" : "twoshot");
           }
           return tag;
-        }, ts, ts, {}, false, bytes);
+        }, ts, ts, {}, false, bytes, async_op);
   }
   std::vector<ccl::cpu::ReduceDesc> descs;
   for (auto& t : ts) descs.push_back(cpu_reduce_desc(rop, t.scalar_type(), W));
@@ -650,7 +651,8 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::allreduce(std::vector<at::Tensor>& ten
   TORCH_CHECK(!opts.sparseIndices.has_value(), "ccl: sparse allreduce is not supported");
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::allreduce", to_ivalues(tensors));
   CCL_OP_PROLOGUE("allreduce", tensors[0], "", tensors_str(tensors), nbytes(tensors))
-  auto w = allreduce_impl(*this, tensors, opts.reduceOp, opTimeout(opts.timeout), OpType::ALLREDUCE, on_cuda, seq, flight__, bytes__,
+  const bool async_op = issuedAsync(opts.asyncOp);
+  auto w = allreduce_impl(*this, tensors, opts.reduceOp, opTimeout(opts.timeout), OpType::ALLREDUCE, on_cuda, seq, flight__, bytes__, async_op,
       [&](std::function<void(ccl::cpu::ShmComm&)> fn, std::vector<at::Tensor> outs) {
         return enqueueCpu(OpType::ALLREDUCE, "oneccl_bindings_for_pytorch::cpu::allreduce", std::move(fn), std::move(outs), {}, false, seq, flight__);
       });
@@ -663,7 +665,8 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::allreduce_coalesced(std::vector<at::Te
   ccl::check_same_type(tensors[0], tensors);
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::allreduce_coalesced", to_ivalues(tensors));
   CCL_OP_PROLOGUE("allreduce_coalesced", tensors[0], "", tensors_str(tensors), nbytes(tensors))
-  auto w = allreduce_impl(*this, tensors, opts.reduceOp, opTimeout(opts.timeout), OpType::ALLREDUCE_COALESCED, on_cuda, seq, flight__, bytes__,
+  const bool async_op = issuedAsync(opts.asyncOp);
+  auto w = allreduce_impl(*this, tensors, opts.reduceOp, opTimeout(opts.timeout), OpType::ALLREDUCE_COALESCED, on_cuda, seq, flight__, bytes__, async_op,
       [&](std::function<void(ccl::cpu::ShmComm&)> fn, std::vector<at::Tensor> outs) {
         return enqueueCpu(OpType::ALLREDUCE_COALESCED, "oneccl_bindings_for_pytorch::cpu::allreduce_coalesced", std::move(fn), std::move(outs), {}, false, seq, flight__);
       });
@@ -679,6 +682,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::reduce(std::vector<at::Tensor>& tensor
   ccl::check_single_tensor(tensors);
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::reduce", to_ivalues(tensors));
   CCL_OP_PROLOGUE("reduce", tensors[0], flow_str(rank_, (int)opts.rootRank), tensors_str(tensors), nbytes(tensors))
+  const bool async_op = issuedAsync(opts.asyncOp);
   at::Tensor t = tensors[0];
   const int root = (int)opts.rootRank;
   const auto tmo = opTimeout(opts.timeout);
@@ -696,7 +700,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::reduce(std::vector<at::Tensor>& tensor
           fill_reduce(a, spec, t.scalar_type());
           C10_CUDA_CHECK(c.reduce(ccl_py::to_ccl_dtype(t.scalar_type()), {a}, s));
           return std::string("twoshot");
-        }, {t}, {t}, {}, false, bytes__);
+        }, {t}, {t}, {}, false, bytes__, async_op);
   } else {
     const auto desc = cpu_reduce_desc(opts.reduceOp, t.scalar_type(), size_);
     w = enqueueCpu(OpType::REDUCE, "oneccl_bindings_for_pytorch::cpu::reduce",
@@ -712,7 +716,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::reduce(std::vector<at::Tensor>& tensor
 // ------------------------------------------------------------------------------------------
 static c10::intrusive_ptr<Work> allgather_pieces(ProcessGroupCCL& pg, OpType type, const char* title_cuda, const char* title_cpu,
     std::vector<at::Tensor> ins, std::vector<std::vector<at::Tensor>> outs, bool nested_result,
-    std::vector<at::Tensor> flat_result, std::chrono::milliseconds tmo, bool on_cuda, uint64_t seq, size_t flight, uint64_t bytes,
+    std::vector<at::Tensor> flat_result, std::chrono::milliseconds tmo, bool on_cuda, uint64_t seq, size_t flight, uint64_t bytes, bool async_op,
     const std::function<c10::intrusive_ptr<Work>(std::function<void(ccl::cpu::ShmComm&)>)>& cpu_enqueue) {
   if (on_cuda) {
     std::vector<at::Tensor> keep = ins;
@@ -754,7 +758,7 @@ static c10::intrusive_ptr<Work> allgather_pieces(ProcessGroupCCL& pg, OpType typ
             C10_CUDA_CHECK(c.all_gather({a}, s));
           }
           return std::string("all_gather");
-        }, keep, nested_result ? std::vector<at::Tensor>{} : flat_result, nested_result ? outs : std::vector<std::vector<at::Tensor>>{}, nested_result, bytes);
+        }, keep, nested_result ? std::vector<at::Tensor>{} : flat_result, nested_result ? outs : std::vector<std::vector<at::Tensor>>{}, nested_result, bytes, async_op);
   }
   return cpu_enqueue([ins, outs, tmo](ccl::cpu::ShmComm& c) {
     for (size_t i = 0; i < ins.size(); ++i) {
@@ -778,9 +782,10 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::allgather(std::vector<std::vector<at::
   TORCH_CHECK(outputTensors[0][rank_].numel() == inputTensors[0].numel(), "allgather: send and recv count doesn't match");
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::allgather", to_ivalues(inputTensors));
   CCL_OP_PROLOGUE("allgather", inputTensors[0], "", tensors_str2(outputTensors, inputTensors), nbytes(outputTensors[0]))
+  const bool async_op = issuedAsync(opts.asyncOp);
   auto outs = outputTensors;
   auto w = allgather_pieces(*this, OpType::ALLGATHER, "oneccl_bindings_for_pytorch::cuda::allgather", "oneccl_bindings_for_pytorch::cpu::allgather",
-      inputTensors, outs, true, {}, opTimeout(opts.timeout), on_cuda, seq, flight__, bytes__,
+      inputTensors, outs, true, {}, opTimeout(opts.timeout), on_cuda, seq, flight__, bytes__, async_op,
       [&](std::function<void(ccl::cpu::ShmComm&)> fn) {
         return enqueueCpu(OpType::ALLGATHER, "oneccl_bindings_for_pytorch::cpu::allgather", std::move(fn), {}, outs, true, seq, flight__);
       });
@@ -803,6 +808,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::_allgather_base(at::Tensor& outputBuff
   TORCH_CHECK(inputBuffer.numel() * size_ == outputBuffer.numel(), "output tensor size must be equal to world_size times input tensor size");
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::_allgather_base", std::vector<c10::IValue>({inputBuffer}));
   CCL_OP_PROLOGUE("_allgather_base", inputBuffer, "", tensors_str(inputBuffer), (uint64_t)outputBuffer.numel() * outputBuffer.element_size())
+  const bool async_op = issuedAsync(opts.asyncOp);
   if (on_cuda) {
     // flat buffers: piece p of the output is at p * bytes, no per-piece tensors are needed
     at::Tensor in = inputBuffer, ob = outputBuffer;
@@ -823,7 +829,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::_allgather_base(at::Tensor& outputBuff
           }
           C10_CUDA_CHECK(c.all_gather({a}, s));
           return std::string("all_gather");
-        }, {in, ob}, {ob}, {}, false, bytes__);
+        }, {in, ob}, {ob}, {}, false, bytes__, async_op);
     CCL_TRACK_COALESCED(w);
     return w;
   }
@@ -831,7 +837,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::_allgather_base(at::Tensor& outputBuff
   std::vector<std::vector<at::Tensor>> outs{split_flat(outputBuffer, size_)};
   at::Tensor ob = outputBuffer;
   auto w = allgather_pieces(*this, OpType::_ALLGATHER_BASE, "oneccl_bindings_for_pytorch::cuda::_allgather_base", "oneccl_bindings_for_pytorch::cpu::_allgather_base",
-      ins, outs, false, {ob}, opTimeout(opts.timeout), on_cuda, seq, flight__, bytes__,
+      ins, outs, false, {ob}, opTimeout(opts.timeout), on_cuda, seq, flight__, bytes__, async_op,
       [&](std::function<void(ccl::cpu::ShmComm&)> fn) {
         return enqueueCpu(OpType::_ALLGATHER_BASE, "oneccl_bindings_for_pytorch::cpu::_allgather_base", std::move(fn), {ob}, {}, false, seq, flight__);
       });
@@ -853,11 +859,12 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::allgather_into_tensor_coalesced(std::v
   }
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::allgather_into_tensor_coalesced", to_ivalues(inputs));
   CCL_OP_PROLOGUE("allgather_into_tensor_coalesced", inputs[0], "", tensors_str(inputs), nbytes(outputs))
+  const bool async_op = issuedAsync(opts.asyncOp);
   std::vector<std::vector<at::Tensor>> outs;
   for (auto& o : outputs) outs.push_back(split_flat(o, size_));
   auto flat = outputs;
   auto w = allgather_pieces(*this, OpType::COALESCED, "oneccl_bindings_for_pytorch::cuda::allgather_into_tensor_coalesced", "",
-      inputs, outs, false, flat, opTimeout(opts.timeout), on_cuda, seq, flight__, bytes__,
+      inputs, outs, false, flat, opTimeout(opts.timeout), on_cuda, seq, flight__, bytes__, async_op,
       [&](std::function<void(ccl::cpu::ShmComm&)> fn) {
         return enqueueCpu(OpType::COALESCED, "oneccl_bindings_for_pytorch::cpu::allgather_into_tensor_coalesced", std::move(fn), flat, {}, false, seq, flight__);
       });
@@ -883,6 +890,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::gather(std::vector<std::vector<at::Ten
   }
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::gather", to_ivalues(inputTensors));
   CCL_OP_PROLOGUE("gather", inputTensors[0], flow_str(rank_, root), tensors_str(inputTensors), nbytes(inputTensors))
+  const bool async_op = issuedAsync(opts.asyncOp);
   at::Tensor in = inputTensors[0];
   std::vector<at::Tensor> outs = rank_ == root ? outputTensors[0] : std::vector<at::Tensor>{};
   const auto tmo = opTimeout(opts.timeout);
@@ -907,7 +915,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::gather(std::vector<std::vector<at::Ten
           if (me == root) for (int p = 0; p < c.world(); ++p) a.out_piece[p] = outs[p].data_ptr();
           C10_CUDA_CHECK(c.rooted({a}, s));
           return std::string("rooted");
-        }, keep, {}, nested, true, bytes__);
+        }, keep, {}, nested, true, bytes__, async_op);
   }
   return enqueueCpu(OpType::GATHER, "oneccl_bindings_for_pytorch::cpu::gather",
       [in, outs, root, tmo](ccl::cpu::ShmComm& c) {
@@ -932,6 +940,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::scatter(std::vector<at::Tensor>& outpu
   }
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::scatter", to_ivalues(outputTensors));
   CCL_OP_PROLOGUE("scatter", outputTensors[0], flow_str(root, rank_), tensors_str(outputTensors), nbytes(outputTensors))
+  const bool async_op = issuedAsync(opts.asyncOp);
   at::Tensor out = outputTensors[0];
   std::vector<at::Tensor> ins = rank_ == root ? inputTensors[0] : std::vector<at::Tensor>{};
   const auto tmo = opTimeout(opts.timeout);
@@ -955,7 +964,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::scatter(std::vector<at::Tensor>& outpu
           if (me == root) for (int p = 0; p < c.world(); ++p) a.in_piece[p] = ins[p].data_ptr();
           C10_CUDA_CHECK(c.rooted({a}, s));
           return std::string("rooted");
-        }, keep, {out}, {}, false, bytes__);
+        }, keep, {out}, {}, false, bytes__, async_op);
   }
   return enqueueCpu(OpType::SCATTER, "oneccl_bindings_for_pytorch::cpu::scatter",
       [out, ins, root, tmo](ccl::cpu::ShmComm& c) {
@@ -970,7 +979,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::scatter(std::vector<at::Tensor>& outpu
 // ------------------------------------------------------------------------------------------
 static c10::intrusive_ptr<Work> reduce_scatter_pieces(ProcessGroupCCL& pg, OpType type, const char* title_cuda,
     std::vector<std::vector<at::Tensor>> ins, std::vector<at::Tensor> outs, const ReduceOp& rop, std::chrono::milliseconds tmo,
-    bool on_cuda, uint64_t bytes, const std::function<c10::intrusive_ptr<Work>(std::function<void(ccl::cpu::ShmComm&)>)>& cpu_enqueue) {
+    bool on_cuda, uint64_t bytes, bool async_op, const std::function<c10::intrusive_ptr<Work>(std::function<void(ccl::cpu::ShmComm&)>)>& cpu_enqueue) {
   const int W = pg.getSize();
   if (on_cuda) {
     std::vector<at::Tensor> keep = outs;
@@ -1027,7 +1036,7 @@ static c10::intrusive_ptr<Work> reduce_scatter_pieces(ProcessGroupCCL& pg, OpTyp
             C10_CUDA_CHECK(c.reduce_scatter(dt, dt, {a}, s));
           }
           return std::string("reduce_scatter");
-        }, keep, outs, {}, false, bytes);
+        }, keep, outs, {}, false, bytes, async_op);
   }
   std::vector<ccl::cpu::ReduceDesc> descs;
   for (auto& o : outs) descs.push_back(cpu_reduce_desc(rop, o.scalar_type(), W));
@@ -1052,9 +1061,10 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::reduce_scatter(std::vector<at::Tensor>
   TORCH_CHECK(inputTensors[0][rank_].numel() == outputTensors[0].numel(), "reduce_scatter: input piece of this rank and output size don't match");
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::reduce_scatter", to_ivalues(outputTensors));
   CCL_OP_PROLOGUE("reduce_scatter", outputTensors[0], "", tensors_str(outputTensors), nbytes(inputTensors[0]))
+  const bool async_op = issuedAsync(opts.asyncOp);
   auto outs = outputTensors;
   auto w = reduce_scatter_pieces(*this, OpType::REDUCE_SCATTER, "oneccl_bindings_for_pytorch::cuda::reduce_scatter", inputTensors, outs, opts.reduceOp,
-      opTimeout(opts.timeout), on_cuda, bytes__,
+      opTimeout(opts.timeout), on_cuda, bytes__, async_op,
       [&](std::function<void(ccl::cpu::ShmComm&)> fn) {
         return enqueueCpu(OpType::REDUCE_SCATTER, "oneccl_bindings_for_pytorch::cpu::reduce_scatter", std::move(fn), outs, {}, false, seq, flight__);
       });
@@ -1069,6 +1079,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::_reduce_scatter_base(at::Tensor& outpu
   TORCH_CHECK(outputBuffer.numel() * size_ == inputBuffer.numel(), "input tensor size must be equal to world_size times output tensor size");
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::_reduce_scatter_base", std::vector<c10::IValue>({inputBuffer}));
   CCL_OP_PROLOGUE("_reduce_scatter_base", inputBuffer, "", tensors_str(inputBuffer), (uint64_t)inputBuffer.numel() * inputBuffer.element_size())
+  const bool async_op = issuedAsync(opts.asyncOp);
   if (on_cuda) {
     at::Tensor in = inputBuffer, ob = outputBuffer;
     const ccl::ReduceSpec spec = ccl::make_reduce_spec(opts.reduceOp, ob.scalar_type(), size_);
@@ -1095,14 +1106,14 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::_reduce_scatter_base(at::Tensor& outpu
           const int dt = ccl_py::to_ccl_dtype(ob.scalar_type());
           C10_CUDA_CHECK(c.reduce_scatter(dt, dt, {a}, s));
           return std::string("reduce_scatter");
-        }, {in, ob}, {ob}, {}, false, bytes__);
+        }, {in, ob}, {ob}, {}, false, bytes__, async_op);
     CCL_TRACK_COALESCED(w);
     return w;
   }
   std::vector<std::vector<at::Tensor>> ins{split_flat(inputBuffer, size_)};
   std::vector<at::Tensor> outs{outputBuffer};
   auto w = reduce_scatter_pieces(*this, OpType::_REDUCE_SCATTER_BASE, "oneccl_bindings_for_pytorch::cuda::_reduce_scatter_base", ins, outs, opts.reduceOp,
-      opTimeout(opts.timeout), on_cuda, bytes__,
+      opTimeout(opts.timeout), on_cuda, bytes__, async_op,
       [&](std::function<void(ccl::cpu::ShmComm&)> fn) {
         return enqueueCpu(OpType::_REDUCE_SCATTER_BASE, "oneccl_bindings_for_pytorch::cpu::_reduce_scatter_base", std::move(fn), outs, {}, false, seq, flight__);
       });
@@ -1122,9 +1133,10 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::reduce_scatter_tensor_coalesced(std::v
   }
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::reduce_scatter_tensor_coalesced", to_ivalues(inputs));
   CCL_OP_PROLOGUE("reduce_scatter_tensor_coalesced", inputs[0], "", tensors_str(inputs), nbytes(inputs))
+  const bool async_op = issuedAsync(opts.asyncOp);
   auto outs = outputs;
   auto w = reduce_scatter_pieces(*this, OpType::COALESCED, "oneccl_bindings_for_pytorch::cuda::reduce_scatter_tensor_coalesced", ins, outs, opts.reduceOp,
-      opTimeout(opts.timeout), on_cuda, bytes__,
+      opTimeout(opts.timeout), on_cuda, bytes__, async_op,
       [&](std::function<void(ccl::cpu::ShmComm&)> fn) {
         return enqueueCpu(OpType::COALESCED, "oneccl_bindings_for_pytorch::cpu::reduce_scatter_tensor_coalesced", std::move(fn), outs, {}, false, seq, flight__);
       });
@@ -1137,7 +1149,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::reduce_scatter_tensor_coalesced(std::v
 // ------------------------------------------------------------------------------------------
 static c10::intrusive_ptr<Work> alltoall_pieces(ProcessGroupCCL& pg, OpType type, const char* title_cuda,
     std::vector<at::Tensor> ins, std::vector<at::Tensor> outs, bool uneven, std::vector<at::Tensor> result,
-    std::chrono::milliseconds tmo, bool on_cuda, uint64_t bytes, const at::Device& dev,
+    std::chrono::milliseconds tmo, bool on_cuda, uint64_t bytes, bool async_op, const at::Device& dev,
     const std::function<c10::intrusive_ptr<Work>(std::function<void(ccl::cpu::ShmComm&)>)>& cpu_enqueue) {
   if (on_cuda) {
     std::vector<at::Tensor> keep = ins;
@@ -1158,7 +1170,7 @@ static c10::intrusive_ptr<Work> alltoall_pieces(ProcessGroupCCL& pg, OpType type
           }
           C10_CUDA_CHECK(c.all_to_all({a}, uneven, s));
           return std::string(uneven ? "all_to_allv" : "all_to_all");
-        }, keep, result, {}, false, bytes);
+        }, keep, result, {}, false, bytes, async_op);
   }
   return cpu_enqueue([ins, outs, tmo](ccl::cpu::ShmComm& c) {
     std::vector<const void*> i(c.world());
@@ -1203,6 +1215,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::alltoall_base(at::Tensor& outputTensor
   ccl::check_split_sizes(outputSplitSizes, outputTensor, size_);
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::alltoall_base", std::vector<c10::IValue>({inputTensor}));
   CCL_OP_PROLOGUE("alltoall_base", inputTensor, "", tensors_str(inputTensor), (uint64_t)inputTensor.numel() * inputTensor.element_size())
+  const bool async_op = issuedAsync(opts.asyncOp);
   // On CUDA the form of the call selects the device protocol: without split lists the fixed-size exchange, with
   // them the one that first agrees on sizes. The choice is made from this rank's arguments alone, so either every
   // rank of the group passes split lists or none does; CCL_DEBUG_CHECKS=1 compares the form across ranks and
@@ -1229,13 +1242,13 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::alltoall_base(at::Tensor& outputTensor
           }
           C10_CUDA_CHECK(c.all_to_all({a}, false, s));
           return std::string("all_to_all");
-        }, {in, ot2}, {ot2}, {}, false, bytes__);
+        }, {in, ot2}, {ot2}, {}, false, bytes__, async_op);
   }
   auto ins = split_rows(inputTensor, inputSplitSizes, size_);
   auto outs = split_rows(outputTensor, outputSplitSizes, size_);
   at::Tensor ot = outputTensor;
   return alltoall_pieces(*this, OpType::ALLTOALL_BASE, "oneccl_bindings_for_pytorch::cuda::alltoall_base", ins, outs, uneven, {ot},
-      opTimeout(opts.timeout), on_cuda, bytes__, inputTensor.device(),
+      opTimeout(opts.timeout), on_cuda, bytes__, async_op, inputTensor.device(),
       [&](std::function<void(ccl::cpu::ShmComm&)> fn) {
         return enqueueCpu(OpType::ALLTOALL_BASE, "oneccl_bindings_for_pytorch::cpu::alltoall_base", std::move(fn), {ot}, {}, false, seq, flight__);
       });
@@ -1248,9 +1261,10 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::alltoall(std::vector<at::Tensor>& outp
   ccl::check_same_type(inputTensors[0], outputTensors);
   RECORD_FUNCTION("oneccl_bindings_for_pytorch::alltoall", to_ivalues(inputTensors));
   CCL_OP_PROLOGUE("alltoall", inputTensors[0], "", tensors_str(inputTensors), nbytes(inputTensors))
+  const bool async_op = issuedAsync(opts.asyncOp);
   auto outs = outputTensors;
   return alltoall_pieces(*this, OpType::ALLTOALL, "oneccl_bindings_for_pytorch::cuda::alltoall", inputTensors, outs, true, outs,
-      opTimeout(opts.timeout), on_cuda, bytes__, inputTensors[0].device(),
+      opTimeout(opts.timeout), on_cuda, bytes__, async_op, inputTensors[0].device(),
       [&](std::function<void(ccl::cpu::ShmComm&)> fn) {
         return enqueueCpu(OpType::ALLTOALL, "oneccl_bindings_for_pytorch::cpu::alltoall", std::move(fn), outs, {}, false, seq, flight__);
       });
@@ -1319,7 +1333,7 @@ c10::intrusive_ptr<Work> ProcessGroupCCL::barrier(const BarrierOptions& opts) {
         [](ccl::CudaComm& c, cudaStream_t s) {
           if (c.world() > 1) C10_CUDA_CHECK(c.barrier(s));
           return std::string("barrier");
-        }, {}, {}, {}, false, 0, /*host_blocking=*/true);
+        }, {}, {}, {}, false, 0, /*async_op=*/true, /*host_blocking=*/true);
   }
   const auto tmo = opTimeout(opts.timeout);
   return enqueueCpu(OpType::BARRIER, "oneccl_bindings_for_pytorch::cpu::barrier",

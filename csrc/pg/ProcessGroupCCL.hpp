@@ -65,6 +65,13 @@ class ProcessGroupCCL : public Backend {
 
     size_t flight_slot = 0;
 
+    // Called when the last owner lets go while the watchdog still knows the work weakly: the tensors go now.
+    void release_resources() override {
+      outputs_.clear();
+      nested_outputs_.clear();
+      future_.reset();
+    }
+
    protected:
     void makeFuture(bool nested, const std::vector<c10::Device>& devices);
     virtual void completeFutureNow();  // marks future_ completed with the outputs
@@ -149,6 +156,8 @@ class ProcessGroupCCL : public Backend {
   uint64_t nextSeq() { return seq_.fetch_add(1); }
   void debugConsistencyCheck(const char* op, at::ScalarType dtype, uint64_t bytes);
   bool timingEnabled() const { return timing_enabled_; }
+  // Inside a coalescing window every op goes to the communication stream: the Work of the window is recorded there.
+  bool issuedAsync(bool asked) const { return asked || coalescing_depth_ > 0; }
 
  private:
   ccl::cpu::ShmComm& shm();
