@@ -1,9 +1,11 @@
 // Host launcher of the tcgen05 bf16 GEMM: builds (and caches) the TMA tensor maps, picks tile
 // width / pipeline depth / split-K cluster size, and launches the kernel from gemm_tcgen05.cuh.
 #include "gemm.h"
+#include "gemm_2sm.cuh"
 #include "gemm_tcgen05.cuh"
 #include "tma_desc.h"
 
+#include <algorithm>
 #include <atomic>
 #include <cstdio>
 #include <cstdlib>
@@ -41,48 +43,110 @@ __global__ void __launch_bounds__(kThreads, 1)
   gemm_tile_body<BN, DUAL>(&tma_a, &tma_b, p, StoreEpilogue<OutT>{}, TileCoord{m0, m0, (int)blockIdx.y * BN});
 }
 
-template <int BN, typename OutT>
-__global__ void __launch_bounds__(kThreads, 1)
-    gemm_persistent_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ CUtensorMap tma_b,
-                           const Params p) {
-  gemm_persistent_body<BN>(&tma_a, &tma_b, p, StoreEpilogue<OutT>{});
+// Operands of the row-major problem D[M, N] = A · B^T for the CTA-pair kernel.
+struct Desc2 {
+  const void *a, *b;
+  int64_t M, N, K, lda, ldb;
+  int b_tiled;
+  int64_t b_packed_rows;
+};
+
+// Tile width for the CTA-pair kernel.
+int pick_bn(int64_t M, int64_t N, int64_t K, bool dual, bool packed) {
+  (void)K;
+  const int64_t mt = (M + 2 * kBM - 1) / (2 * kBM);
+  double best = 1e30;
+  int bn = 256;
+  for (int w = 256; w >= 64; w -= (packed ? w / 2 : 32)) {
+    const int64_t cols = dual ? w / 2 : w;
+    if (dual && cols % 32 != 0) continue;
+    const int64_t nt = (N + cols - 1) / cols;
+    const int64_t waves = (mt * nt + 73) / 74;
+    const double cost = (double)waves * std::max(2.0 * w, 256.0 + w);
+    if (cost < best * 0.999) {
+      best = cost;
+      bn = w;
+    }
+  }
+  return bn;
 }
 
-// Compute-bound shapes: persistent CTAs, double-buffered TMEM accumulators.
-template <int BN, typename OutT>
-cudaError_t launch_persistent(const GemmDesc& d, cudaStream_t stream) {
-  const int m_tiles = (int)((d.M + kBM - 1) / kBM);
-  const int n_tiles = (int)((d.N + BN - 1) / BN);
-  constexpr size_t kSmemMax = 200 * 1024;
-  int stages = kMaxStages;
-  while (stages > 2 && persistent_smem_bytes<BN>(stages) > kSmemMax) --stages;
-  const size_t smem = persistent_smem_bytes<BN>(stages);
-  CUtensorMap ta, tb;
-  if (!tma::make_2d_bf16(&ta, d.a, (uint64_t)d.M, (uint64_t)d.K, (uint64_t)d.lda, kBM, kBK)) return cudaErrorInvalidValue;
-  if (!tma::make_2d_bf16(&tb, d.b, (uint64_t)d.N, (uint64_t)d.K, (uint64_t)d.ldb, BN, kBK)) return cudaErrorInvalidValue;
-  Params p{};
-  p.M = (int)d.M;
-  p.N = (int)d.N;
-  p.K = (int)d.K;
+template <bool DUAL, typename OutT>
+cudaError_t launch_2sm(const GemmDesc& d, const Desc2& q, int bn, cudaStream_t stream) {
+  Params2 p{};
+  p.M = (int)q.M;
+  p.N = (int)q.N;
+  p.K = (int)q.K;
+  p.bn = bn;
+  const int k_iters = (int)((q.K + kBK - 1) / kBK);
+  p.m_tiles = (int)((q.M + 2 * kBM - 1) / (2 * kBM));
+  const int cols = DUAL ? bn / 2 : bn;
+  p.n_tiles = (int)((q.N + cols - 1) / cols);
+  p.b_tiled = q.b_tiled;
+  p.k_tiles = k_iters;
+  p.dual_off = (int)d.dual_off;
   p.out = d.out;
   p.ldo = d.ldo;
-  p.stages = stages;
-  p.splitk = 1;
   p.status = d.status;
-  auto kern = gemm_persistent_kernel<BN, OutT>;
+  p.tma_out = (reinterpret_cast<uintptr_t>(d.out) & 15) == 0 && (d.ldo * (int64_t)sizeof(OutT)) % 16 == 0;
+  CUtensorMap ta, tb, to;
+  if (!tma::make_2d_bf16(&ta, q.a, (uint64_t)q.M, (uint64_t)q.K, (uint64_t)q.lda, kBM, kBK)) return cudaErrorInvalidValue;
+  if (q.b_tiled) {
+    if (!tma::make_2d_bf16(&tb, q.b, (uint64_t)q.b_packed_rows, (uint64_t)kBK, (uint64_t)kBK, bn / 2, kBK)) return cudaErrorInvalidValue;
+  } else if (!tma::make_2d_bf16(&tb, q.b, (uint64_t)(DUAL ? d.dual_off + q.N : q.N), (uint64_t)q.K, (uint64_t)q.ldb, bn / 2, kBK)) {
+    return cudaErrorInvalidValue;
+  }
+  if (p.tma_out) {
+    if (!tma::make_2d_result(&to, d.out, (uint64_t)q.M, (uint64_t)q.N, (uint64_t)d.ldo, sizeof(OutT) == 4)) return cudaErrorInvalidValue;
+  } else {
+    to = ta;
+  }
+  auto kern = gemm_2sm_kernel<DUAL, OutT>;
+  const size_t smem = smem_bytes_2sm();
   static DeviceOnce configured;
   if (configured.pending()) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemMax + 2048);
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_bytes_2sm());
     if (e != cudaSuccess) return e;
     configured.done();
   }
-  int sms = 148;
-  const int total = m_tiles * n_tiles;
-  const int grid = total < sms ? total : sms;
-  kern<<<grid, kThreads, smem, stream>>>(ta, tb, p);
-  cudaError_t e = cudaGetLastError();
+  const int total = p.m_tiles * p.n_tiles;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(2 * (total < 74 ? total : 74), 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_launch_attr(&attr[0]);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, ta, tb, to, p);
   if (e == cudaSuccess) g_launches.fetch_add(1);
   return e;
+}
+
+cudaError_t dispatch_2sm(const GemmDesc& d, cudaStream_t stream) {
+  Desc2 q{};
+  q.K = d.K;
+  if (d.trans_out) {  // out[n * ldo + m]: the rows of the result are B's
+    q.a = d.b;
+    q.M = d.N;
+    q.lda = d.ldb;
+    q.b = d.a;
+    q.N = d.M;
+    q.ldb = d.lda;
+    q.b_tiled = d.a_tiled;
+    q.b_packed_rows = d.a_packed_rows;
+  } else {
+    q.a = d.a;
+    q.M = d.M;
+    q.lda = d.lda;
+    q.b = d.b;
+    q.N = d.N;
+    q.ldb = d.ldb;
+  }
+  // a given width counts result columns (dual: of each half)
+  int bn = d.bn > 0 ? std::min(256, d.dual_off > 0 ? 2 * d.bn : d.bn) : pick_bn(q.M, q.N, q.K, d.dual_off > 0, q.b_tiled != 0);
+  if (d.dual_off > 0) return d.out_fp32 ? launch_2sm<true, float>(d, q, bn, stream) : launch_2sm<true, __nv_bfloat16>(d, q, bn, stream);
+  return d.out_fp32 ? launch_2sm<false, float>(d, q, bn, stream) : launch_2sm<false, __nv_bfloat16>(d, q, bn, stream);
 }
 
 // Pipeline depth for a given split: narrow (decode) tiles are memory-bound, so when one CTA per SM
@@ -193,6 +257,11 @@ cudaError_t gemm_bf16_tn(const GemmDesc& d, cudaStream_t stream) {
   if ((!d.a_tiled && (d.lda % 8)) || (d.ldb % 8)) return cudaErrorInvalidValue;  // TMA strides: 16-byte multiples
   if ((reinterpret_cast<uintptr_t>(d.a) & 15) || (reinterpret_cast<uintptr_t>(d.b) & 15))
     return cudaErrorInvalidValue;
+  // Many result rows: the CTA-pair kernel, whose result is row-major (with trans_out the rows are B's; a dual or packed A
+  // can only be its B operand, so those need trans_out).
+  const bool width_ok = d.bn == 0 || d.bn == 64 || d.bn == 128 || d.bn == 256 || (d.bn > 64 && d.bn < 256 && d.bn % 32 == 0 && !d.a_tiled && d.dual_off == 0);
+  if (width_ok && d.splitk <= 1 && (d.trans_out ? d.N : d.M) > 128 && (d.trans_out || (!d.a_tiled && d.dual_off == 0)))
+    return gemm::dispatch_2sm(d, stream);
   int bn = d.bn;
   if (bn == 0) {
     if (d.N <= 16) bn = 16;
@@ -224,13 +293,6 @@ cudaError_t gemm_bf16_tn(const GemmDesc& d, cudaStream_t stream) {
       if (splitk > 4) splitk = 4;
       if (splitk < 1) splitk = 1;
     }
-  }
-  // large row-major problems without split-K: the persistent kernel
-  if (!d.a_tiled && !d.trans_out && d.dual_off == 0 && splitk == 1 && (bn == 128 || bn == 256) && !d.no_persistent &&
-      ((d.M + 127) / 128) * ((d.N + bn - 1) / bn) >= 148) {
-    if (bn == 256)
-      return d.out_fp32 ? gemm::launch_persistent<256, float>(d, stream) : gemm::launch_persistent<256, __nv_bfloat16>(d, stream);
-    return d.out_fp32 ? gemm::launch_persistent<128, float>(d, stream) : gemm::launch_persistent<128, __nv_bfloat16>(d, stream);
   }
   switch (bn) {
     case 16: return gemm::dispatch_bn<16>(d, splitk, stream);

@@ -46,7 +46,6 @@ struct GemmDesc {
   // second operand starts dual_off (a multiple of 128) packed rows after the first.
   int a_tiled = 0;
   int64_t a_packed_rows = 0;  // total rows of the packed [*, 64] matrix
-  int no_persistent = 0;  // 1: force the one-tile-per-CTA kernel (testing)
   int* status = nullptr;  // optional device error word
 };
 

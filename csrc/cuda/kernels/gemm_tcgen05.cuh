@@ -198,34 +198,33 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap* tma_a, const C
   const uint32_t tmem_base = bars->tmem_base;
   ptx::griddep_launch_dependents();
 
+  // The two issuing loops are chains of one thread. Electing it (rather than testing lane == 0) tells the compiler that one
+  // thread runs them: without that every tcgen05.mma and TMA instruction was wrapped in a loop over the active lanes, some
+  // 500 clocks per K step. For the same reason the ring is walked with counters and the descriptors by addition.
   if (warp == 0) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       ptx::prefetch_tmap(tma_a);
       ptx::prefetch_tmap(tma_b);
       if (p.acquire_a) asm volatile("fence.proxy.async;" ::: "memory");
-      auto load_a = [&](int i) {
-        const int s = i % stages;
-        uint8_t* st = smem + (size_t)s * kStage;
-        const int kx = (it_begin + i) * kBK;
+      // TMA coordinates of K step i of this split: packed tiles follow each other kBM rows apart
+      const int ax_step = p.a_tiled ? 0 : kBK, ay_step = p.a_tiled ? kBM : 0;
+      const int kx0 = it_begin * kBK;
+      int ax = p.a_tiled ? 0 : kx0;
+      int ay = p.a_tiled ? ((tc.a_row / kBM) * p.k_tiles + it_begin) * kBM : tc.a_row;
+      const int dual_rows = p.a_tiled ? (p.dual_off / kBM) * p.k_tiles * kBM : p.dual_off;
+      auto load_a = [&](int s) {
+        uint8_t* st = smem + s * kStage;
         ptx::mbar_arrive_expect_tx(&bars->full[s], kStage);
-        if (p.a_tiled) {
-          // one contiguous 16 KB tile per load
-          const int kt = it_begin + i;
-          ptx::tma_load_2d(st, tma_a, &bars->full[s], 0, ((tc.a_row / kBM) * p.k_tiles + kt) * kBM);
-          if (DUAL)
-            ptx::tma_load_2d(st + kABytes, tma_a, &bars->full[s], 0,
-                             (((tc.a_row + p.dual_off) / kBM) * p.k_tiles + kt) * kBM);
-        } else {
-          ptx::tma_load_2d(st, tma_a, &bars->full[s], kx, tc.a_row);
-          if (DUAL) ptx::tma_load_2d(st + kABytes, tma_a, &bars->full[s], kx, tc.a_row + p.dual_off);
-        }
+        ptx::tma_load_2d(st, tma_a, &bars->full[s], ax, ay);
+        if (DUAL) ptx::tma_load_2d(st + kABytes, tma_a, &bars->full[s], ax, ay + dual_rows);
+        ax += ax_step;
+        ay += ay_step;
       };
-      auto load_b = [&](int i) {
-        const int s = i % stages;
-        uint8_t* st = smem + (size_t)s * kStage;
-        ptx::tma_load_2d(st + kABytes * (DUAL ? 2 : 1), tma_b, &bars->full[s], (it_begin + i) * kBK, n0);
+      auto load_b = [&](int s, int i) {
+        ptx::tma_load_2d(smem + s * kStage + kABytes * (DUAL ? 2 : 1), tma_b, &bars->full[s], kx0 + i * kBK, n0);
       };
-      int i0 = 0;
+      int i0 = 0, s = 0;
+      uint32_t phase = 1;  // the first pass over the ring finds it empty
       if (p.a_static) {
         // A (weights) is not produced by any earlier kernel: fill the pipeline with A tiles while
         // the predecessor kernel is still running, then wait for it and fetch the B tiles.
@@ -243,49 +242,53 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap* tma_a, const C
           }
         }
         ptx::griddep_wait();
-        for (int i = 0; i < pre; ++i) load_b(i);
+        for (int i = 0; i < pre; ++i) load_b(i, i);
         i0 = pre;
+        if (pre == stages) phase = 0;
+        else s = pre;
       } else {
         ptx::griddep_wait();
       }
       for (int i = i0; i < n_iters; ++i) {
-        const int s = i % stages;
-        const uint32_t ph = (i / stages) & 1;
-        if (!ptx::mbar_wait(&bars->empty[s], ph ^ 1)) {
+        if (!ptx::mbar_wait(&bars->empty[s], phase)) {
           bars->failed = 1;
           if (p.status) atomicExch(p.status, 101);
           break;
         }
-        load_a(i);
-        load_b(i);
+        load_a(s);
+        load_b(s, i);
+        if (++s == stages) {
+          s = 0;
+          phase ^= 1;
+        }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       constexpr uint32_t idesc = ptx::make_idesc_bf16(kBM, BN);
-      bool ok = true;
-      for (int i = 0; i < n_iters && ok; ++i) {
-        const int s = i % stages;
-        const uint32_t ph = (i / stages) & 1;
-        if (!ptx::mbar_wait(&bars->full[s], ph)) {
+      const uint64_t desc_a0 = ptx::make_desc_sw128(ptx::smem_u32(smem));
+      int s = 0;
+      uint32_t phase = 0;
+      for (int i = 0; i < n_iters; ++i) {
+        if (!ptx::mbar_wait(&bars->full[s], phase)) {
           bars->failed = 1;
           if (p.status) atomicExch(p.status, 102);
-          ok = false;
           break;
         }
         ptx::tc_fence_after();
-        const uint32_t a_addr = ptx::smem_u32(smem + (size_t)s * kStage);
-        const uint32_t b_addr = a_addr + kABytes * (DUAL ? 2 : 1);
+        const uint64_t da = desc_a0 + (uint32_t)(s * (kStage >> 4));
+        const uint64_t db = da + (uint32_t)((kABytes * (DUAL ? 2 : 1)) >> 4);
 #pragma unroll
         for (int k = 0; k < kBK / 16; ++k) {
-          const uint64_t db = ptx::make_desc_sw128(b_addr + k * 32);
           const uint32_t acc = (i > 0 || k > 0) ? 1u : 0u;
-          ptx::umma_bf16_ss(tmem_base, ptx::make_desc_sw128(a_addr + k * 32), db, idesc, acc);
-          if (DUAL)
-            ptx::umma_bf16_ss(tmem_base + BN, ptx::make_desc_sw128(a_addr + kABytes + k * 32), db,
-                              idesc, acc);
+          ptx::umma_bf16_ss(tmem_base, da + k * 2, db + k * 2, idesc, acc);
+          if (DUAL) ptx::umma_bf16_ss(tmem_base + BN, da + (kABytes >> 4) + k * 2, db + k * 2, idesc, acc);
         }
         ptx::umma_commit(&bars->empty[s]);  // frees the stage once these MMAs have read it
+        if (++s == stages) {
+          s = 0;
+          phase ^= 1;
+        }
       }
       ptx::umma_commit(&bars->accum);
     }
@@ -393,172 +396,6 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap* tma_a, const C
     }
   }
 
-  ptx::tc_fence_before();
-  __syncthreads();
-  if (warp == 1) ptx::tmem_dealloc(tmem_base, kTmemCols);
-}
-
-
-// ---------------------------------------------------------------------------------------------
-// Persistent variant for compute-bound problems: one CTA per SM walks a list of output tiles
-// (grouped so that the tiles in flight at any time share A and B panels in L2). The smem ring
-// keeps running across tiles, and the accumulator is double-buffered in TMEM (2 x BN columns):
-// while the epilogue warps drain tile i, the MMA warp already accumulates tile i+1.
-// ---------------------------------------------------------------------------------------------
-struct __align__(8) PersistentBarriers {
-  uint64_t full[kMaxStages];
-  uint64_t empty[kMaxStages];
-  uint64_t tmem_full[2];
-  uint64_t tmem_empty[2];
-  uint32_t tmem_base;
-  uint32_t failed;
-};
-
-template <int BN>
-__host__ __device__ constexpr size_t persistent_smem_bytes(int stages) {
-  return 1024 + (size_t)stages * stage_bytes<BN, false>() + sizeof(PersistentBarriers);
-}
-
-__device__ __forceinline__ void tile_of(int t, int m_tiles, int n_tiles, int& mt, int& nt) {
-  constexpr int kGroupM = 16;
-  const int in_group = kGroupM * n_tiles;
-  const int gid = t / in_group;
-  const int first_m = gid * kGroupM;
-  const int gsm = (m_tiles - first_m) < kGroupM ? (m_tiles - first_m) : kGroupM;
-  const int r = t - gid * in_group;
-  mt = first_m + r % gsm;
-  nt = r / gsm;
-}
-
-template <int BN, typename EpiFn>
-__device__ __forceinline__ void gemm_persistent_body(const CUtensorMap* tma_a, const CUtensorMap* tma_b,
-                                                     const Params& p, const EpiFn& epi) {
-  static_assert(BN == 128 || BN == 256, "persistent kernel: BN 128 or 256 (2*BN TMEM columns)");
-  extern __shared__ uint8_t smem_raw[];
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                             ~uintptr_t(1023));
-  constexpr int kStage = stage_bytes<BN, false>();
-  constexpr int kABytes = kBM * kBK * 2;
-  constexpr uint32_t kTmemCols = 2 * BN;
-  const int stages = p.stages;
-  PersistentBarriers* bars = reinterpret_cast<PersistentBarriers*>(smem + (size_t)stages * kStage);
-  const int warp = threadIdx.x >> 5;
-  const int lane = threadIdx.x & 31;
-  const int m_tiles = (p.M + kBM - 1) / kBM;
-  const int n_tiles = (p.N + BN - 1) / BN;
-  const int total = m_tiles * n_tiles;
-  const int k_iters = (p.K + kBK - 1) / kBK;
-
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < stages; ++s) {
-      ptx::mbar_init(&bars->full[s], 1);
-      ptx::mbar_init(&bars->empty[s], 1);
-    }
-    for (int b = 0; b < 2; ++b) {
-      ptx::mbar_init(&bars->tmem_full[b], 1);
-      ptx::mbar_init(&bars->tmem_empty[b], 128);  // every epilogue thread arrives
-    }
-    bars->failed = 0;
-    ptx::fence_mbar_init();
-  }
-  if (warp == 1) {
-    ptx::tmem_alloc(&bars->tmem_base, kTmemCols);
-    ptx::tmem_relinquish();
-  }
-  ptx::tc_fence_before();
-  __syncthreads();
-  ptx::tc_fence_after();
-  const uint32_t tmem_base = bars->tmem_base;
-
-  if (warp == 0) {
-    if (lane == 0) {
-      ptx::prefetch_tmap(tma_a);
-      ptx::prefetch_tmap(tma_b);
-      uint32_t it = 0;
-      for (int t = blockIdx.x; t < total; t += gridDim.x) {
-        int mt, nt;
-        tile_of(t, m_tiles, n_tiles, mt, nt);
-        for (int k = 0; k < k_iters; ++k, ++it) {
-          const int s = it % stages;
-          const uint32_t ph = (it / stages) & 1;
-          if (!ptx::mbar_wait(&bars->empty[s], ph ^ 1)) {
-            bars->failed = 1;
-            if (p.status) atomicExch(p.status, 111);
-            t = total;
-            break;
-          }
-          uint8_t* st = smem + (size_t)s * kStage;
-          ptx::mbar_arrive_expect_tx(&bars->full[s], kStage);
-          ptx::tma_load_2d(st, tma_a, &bars->full[s], k * kBK, mt * kBM);
-          ptx::tma_load_2d(st + kABytes, tma_b, &bars->full[s], k * kBK, nt * BN);
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (lane == 0) {
-      constexpr uint32_t idesc = ptx::make_idesc_bf16(kBM, BN);
-      uint32_t it = 0;
-      int i = 0;
-      for (int t = blockIdx.x; t < total; t += gridDim.x, ++i) {
-        const int acc = i & 1;
-        if (!ptx::mbar_wait(&bars->tmem_empty[acc], (((uint32_t)i >> 1) & 1) ^ 1)) {
-          bars->failed = 1;
-          if (p.status) atomicExch(p.status, 112);
-          break;
-        }
-        ptx::tc_fence_after();
-        bool ok = true;
-        for (int k = 0; k < k_iters; ++k, ++it) {
-          const int s = it % stages;
-          const uint32_t ph = (it / stages) & 1;
-          if (!ptx::mbar_wait(&bars->full[s], ph)) {
-            bars->failed = 1;
-            if (p.status) atomicExch(p.status, 113);
-            ok = false;
-            break;
-          }
-          ptx::tc_fence_after();
-          const uint32_t a_addr = ptx::smem_u32(smem + (size_t)s * kStage);
-          const uint32_t b_addr = a_addr + kABytes;
-#pragma unroll
-          for (int kk = 0; kk < kBK / 16; ++kk) {
-            ptx::umma_bf16_ss(tmem_base + acc * BN, ptx::make_desc_sw128(a_addr + kk * 32),
-                              ptx::make_desc_sw128(b_addr + kk * 32), idesc, (k > 0 || kk > 0) ? 1u : 0u);
-          }
-          ptx::umma_commit(&bars->empty[s]);
-        }
-        if (!ok) break;
-        ptx::umma_commit(&bars->tmem_full[acc]);
-      }
-    }
-  } else {
-    const int q = warp & 3;
-    const int row = q * 32 + lane;
-    int i = 0;
-    for (int t = blockIdx.x; t < total; t += gridDim.x, ++i) {
-      int mt, nt;
-      tile_of(t, m_tiles, n_tiles, mt, nt);
-      const int acc = i & 1;
-      if (!ptx::mbar_wait(&bars->tmem_full[acc], ((uint32_t)i >> 1) & 1)) {
-        bars->failed = 1;
-        if (p.status) atomicExch(p.status, 114);
-        break;
-      }
-      ptx::tc_fence_after();
-#pragma unroll 2
-      for (int c = 0; c < BN; c += 16) {
-        uint32_t r[16];
-        ptx::tmem_ld_32x32b_x16(tmem_base + ((uint32_t)(q * 32) << 16) + acc * BN + c, r);
-        ptx::tmem_ld_wait();
-        float v[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]);
-        epi(p, mt * kBM + row, nt * BN + c, v);
-      }
-      ptx::tc_fence_before();
-      ptx::mbar_arrive(&bars->tmem_empty[acc]);
-    }
-  }
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == 1) ptx::tmem_dealloc(tmem_base, kTmemCols);

@@ -13,5 +13,8 @@ namespace tma {
 bool make_2d_bf16(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld,
                   uint32_t box_rows, uint32_t box_cols);
 
+// Result matrix of bf16 (64-byte swizzle) or fp32 (128-byte swizzle), stored in blocks of 32 x 32.
+bool make_2d_result(CUtensorMap* out, const void* base, uint64_t rows, uint64_t cols, uint64_t ld, bool fp32);
+
 }  // namespace tma
 }  // namespace ccl

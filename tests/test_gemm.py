@@ -115,3 +115,47 @@ def test_gemm_pretiled_swiglu(batch):
     torch.cuda.synchronize()
     ref = torch.nn.functional.silu(x.float() @ wg.float().t()) * (x.float() @ wu.float().t())
     _check(out, ref, K)
+
+
+@pytest.mark.parametrize("M,N,K,width", [
+    (129, 64, 64, 0),        # one row more than the one-CTA kernel takes, a single K step
+    (256, 32, 72, 64),       # fewer columns than a tile, K not a multiple of the stage
+    (385, 513, 448, 0),      # odd CTA of the last pair without rows; one column in the last tile, unaligned rows
+    (1000, 1003, 520, 128),  # row starts that no TMA store can take
+    (2049, 2500, 328, 96), (2049, 2500, 328, 160), (2049, 2500, 328, 224),
+    (5000, 4100, 1032, 256),  # several tiles per pair: both accumulators, the ring across tiles
+])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_gemm_cta_pairs(M, N, K, width, out_dtype):
+    """Row-major results of more than 128 rows: 256-row tiles on CTA pairs, every tile width and both ways of storing."""
+    torch.manual_seed(6)
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    out = torch.full((M + 1, N), float("nan"), device="cuda", dtype=out_dtype)
+    _C().gemm_bf16_tn(a, b, out[:M], False, 0, 1, width)
+    torch.cuda.synchronize()
+    ref = _ref(a, b)
+    # fp32 sums of exact products in another order: K * 2^-24 of the largest partial sum; bf16 results: half a unit (2^-9)
+    rel = K * 2.0**-24 + (2.0**-9 if out_dtype == torch.bfloat16 else 0.0)
+    assert ((out[:M].float() - ref).norm() / ref.norm()).item() <= rel
+    assert torch.isnan(out[M]).all(), "stored past the last row"
+
+
+@pytest.mark.parametrize("rows,K,tokens", [(64, 64, 129), (1000, 1376, 257), (1536, 512, 1030)])
+@pytest.mark.parametrize("dual", [False, True])
+def test_gemm_cta_pairs_packed(rows, K, tokens, dual):
+    """Pre-tiled weights as the B operand of the CTA-pair kernel, alone and as SwiGLU pairs."""
+    from torch_ccl_b200.ops import pack_weight
+
+    torch.manual_seed(7)
+    w = [torch.randn(rows, K, device="cuda", dtype=torch.bfloat16) * 0.05 for _ in range(2)]
+    x = torch.randn(tokens, K, device="cuda", dtype=torch.bfloat16)
+    out = torch.full((tokens, rows), float("nan"), device="cuda", dtype=torch.bfloat16)
+    if dual:
+        _C().gemm_bf16_tn(torch.cat([pack_weight(t) for t in w]), x, out, True, (rows + 127) // 128 * 128, 1, 0, rows)
+        ref = torch.nn.functional.silu(_ref(x, w[0])) * _ref(x, w[1])
+    else:
+        _C().gemm_bf16_tn(pack_weight(w[0]), x, out, True, 0, 1, 0, rows)
+        ref = _ref(x, w[0])
+    torch.cuda.synchronize()
+    assert ((out.float() - ref).norm() / ref.norm()).item() <= 2.0**-9 + K * 2.0**-22  # silu's __expf adds 2 ulp
