@@ -6,6 +6,7 @@
 #include "bindings/common.h"
 #include "cuda/kernels/decode_attention.h"
 #include "cuda/kernels/gemm.h"
+#include "cuda/kernels/prefill.h"
 
 namespace ccl_py {
 
@@ -55,6 +56,34 @@ void bind_model_ops(py::module& m) {
       },
       py::arg("qkv"), py::arg("k_cache"), py::arg("v_cache"), py::arg("positions"), py::arg("cos"), py::arg("sin"),
       py::arg("out"), py::arg("scratch"), py::arg("counters"), py::arg("n_heads"), py::arg("n_kv_heads"), py::arg("nsplit"));
+  m.def(
+      "rope_append",
+      [](at::Tensor& qkv, at::Tensor& k_cache, at::Tensor& v_cache, const at::Tensor& cos, const at::Tensor& sin, int64_t n_heads, int64_t seq) {
+        TORCH_CHECK(qkv.is_cuda() && qkv.scalar_type() == at::kBFloat16 && qkv.dim() == 2 && qkv.stride(1) == 1, "qkv: [sequences * seq, (h+2kv)*128] bf16");
+        TORCH_CHECK(k_cache.dim() == 4 && k_cache.is_contiguous() && k_cache.scalar_type() == at::kBFloat16 && k_cache.size(3) == 128 &&
+                        v_cache.sizes() == k_cache.sizes() && v_cache.is_contiguous() && v_cache.scalar_type() == at::kBFloat16,
+                    "caches: [sequences, kv_heads, max_seq, 128] bf16");
+        TORCH_CHECK(cos.scalar_type() == at::kFloat && sin.scalar_type() == at::kFloat && cos.is_contiguous() && sin.is_contiguous() &&
+                        cos.size(0) >= seq && sin.size(0) >= seq && cos.size(1) == 64 && sin.size(1) == 64, "cos/sin: [>= seq, 64] fp32");
+        TORCH_CHECK(seq > 0 && qkv.size(0) % seq == 0 && qkv.size(0) / seq <= k_cache.size(0) && seq <= k_cache.size(2), "rope_append: sequences do not fit the cache");
+        TORCH_CHECK(qkv.size(1) >= (n_heads + 2 * k_cache.size(1)) * 128, "qkv row too short");
+        c10::cuda::CUDAGuard g(qkv.device());
+        ccl::RopeAppendParams p;
+        p.qkv = reinterpret_cast<__nv_bfloat16*>(qkv.data_ptr());
+        p.qkv_stride = qkv.stride(0);
+        p.k_cache = reinterpret_cast<__nv_bfloat16*>(k_cache.data_ptr());
+        p.v_cache = reinterpret_cast<__nv_bfloat16*>(v_cache.data_ptr());
+        p.cos = cos.data_ptr<float>();
+        p.sin = sin.data_ptr<float>();
+        p.rows = (int)qkv.size(0);
+        p.seq = (int)seq;
+        p.n_heads = (int)n_heads;
+        p.n_kv_heads = (int)k_cache.size(1);
+        p.max_seq = (int)k_cache.size(2);
+        cudaError_t e = ccl::rope_append(p, c10::cuda::getCurrentCUDAStream());
+        TORCH_CHECK(e == cudaSuccess, "rope_append launch failed: ", cudaGetErrorString(e));
+      },
+      py::arg("qkv"), py::arg("k_cache"), py::arg("v_cache"), py::arg("cos"), py::arg("sin"), py::arg("n_heads"), py::arg("seq"));
 }
 
 }  // namespace ccl_py

@@ -18,6 +18,7 @@
 #include "ll_norm.cuh"
 #include "gemm.h"
 
+#include <algorithm>
 #include <cstdio>
 
 namespace ccl {
@@ -1026,6 +1027,71 @@ __global__ void __launch_bounds__(512) allreduce_residual_rmsnorm_kernel(const _
 }
 
 // ---------------------------------------------------------------------------------------------
+// The same without peers (one-rank communicators: a single GPU, prompts of any length). Bound by memory: five passes of
+// a row's bytes (x, residual in and out, out; the weight stays in cache). One CTA per row; every thread requests its
+// vectors of x and of the residual before it uses one. The kernel above walks 64 rows per CTA, one block barrier after
+// the other, with one or two CTAs per SM: 16384 x 4096 bf16 took 351 us there.
+// ---------------------------------------------------------------------------------------------
+template <typename T, int MV>
+__global__ void __launch_bounds__(512) residual_rmsnorm_kernel(const FusedNormArgs a) {
+  __shared__ float s_red[33];
+  ptx::griddep_launch_dependents();
+  const int hv = a.hidden / 8;
+  const int row = blockIdx.x;
+  Vec<T> wv[MV];
+  ll_load_norm_weight<T, MV>(a.weight, 0, hv, wv);
+  ptx::griddep_wait();
+  const size_t row_bytes = (size_t)a.hidden * sizeof(T);
+  const char* x = static_cast<const char*>(a.x);
+  if (a.gather_tokens) {
+    const long long idx = a.gather_tokens[row] - a.gather_base;
+    x = (idx >= 0 && idx < a.gather_rows) ? x + (size_t)idx * row_bytes : nullptr;
+  } else {
+    x += (size_t)row * row_bytes;
+  }
+  char* res = static_cast<char*>(a.residual) + (size_t)row * row_bytes;
+  Vec<T> xv[MV], hn[MV];
+#pragma unroll
+  for (int k = 0; k < MV; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+    *reinterpret_cast<uint4*>(&xv[k]) = (x && i < hv) ? *reinterpret_cast<const uint4*>(x + (size_t)i * 16) : make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(&hn[k]) = (!a.zero_residual && i < hv) ? *reinterpret_cast<const uint4*>(res + (size_t)i * 16) : make_uint4(0, 0, 0, 0);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < MV; ++k) {
+    const int i = threadIdx.x + k * blockDim.x;
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+      hn[k].v[t] = a.zero_residual ? xv[k].v[t] : ll_round_to<T>(to_acc(xv[k].v[t]) + to_acc(hn[k].v[t]));
+      const float h = to_acc(hn[k].v[t]);
+      ss += h * h;
+    }
+    if (i < hv) *reinterpret_cast<uint4*>(res + (size_t)i * 16) = *reinterpret_cast<const uint4*>(&hn[k]);
+  }
+  const float rstd = rsqrtf(block_sum(ss, s_red) / (float)a.hidden + a.eps);
+  ll_row_write_norm<T, MV>(hn, wv, rstd, 0, hv, static_cast<char*>(a.out) + (size_t)row * row_bytes);
+}
+
+template <typename T>
+cudaError_t launch_residual_rmsnorm(const FusedNormArgs& a, cudaStream_t stream) {
+  // Few rows (decode): one vector per thread, for the shortest chain. Many: four, so that enough CTAs and loads are in
+  // flight on an SM (the crossover is where one CTA per SM of the wide form no longer covers the rows).
+  const int hv = a.hidden / 8;
+  const bool many = a.rows > 4 * 148 || hv > 512;
+  const int mv = many ? 4 : 1;
+  const int threads = std::max(32, ((hv + mv - 1) / mv + 31) / 32 * 32);
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = dim3(a.rows, 1, 1);
+  lc.blockDim = dim3(threads, 1, 1);
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  lc.attrs = attr;
+  lc.numAttrs = pdl_launch_attr(&attr[0]);
+  return many ? cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 4>, a) : cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 1>, a);
+}
+
+// ---------------------------------------------------------------------------------------------
 // launch plumbing
 // ---------------------------------------------------------------------------------------------
 template <typename ArgsT, template <bool> class LT, typename KR, typename KE>
@@ -1133,6 +1199,11 @@ cudaError_t launch_barrier(const RankCtx* ctx, const CollArgs* args, const Launc
   return launch_pair<CollArgs, Launch>(barrier_kernel<false>, barrier_kernel<true>, ctx, args, c);
 }
 cudaError_t launch_allreduce_residual_rmsnorm(int dtype, const RankCtx* ctx, const FusedNormArgs* args, const LaunchCfg& cfg) {
+  if (!cfg.cooperative && ctx->world == 1 && args->ablate == kAblateNone) {
+    if (dtype == kBF16) return launch_residual_rmsnorm<__nv_bfloat16>(*args, cfg.stream);
+    if (dtype == kF16) return launch_residual_rmsnorm<__half>(*args, cfg.stream);
+    return cudaErrorInvalidValue;
+  }
   if (dtype == kBF16)
     return launch_pair<FusedNormArgs, LaunchNorm>(allreduce_residual_rmsnorm_kernel<__nv_bfloat16, false>, allreduce_residual_rmsnorm_kernel<__nv_bfloat16, true>, ctx, args, cfg);
   if (dtype == kF16)

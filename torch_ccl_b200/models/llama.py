@@ -210,6 +210,9 @@ class TPLlamaDecoder:
     def _gemm_t(self, w, x, out, rows, dual=0, splitk=0):
         """out[b, n] = x[b, :] @ W[n, :]^T with the pre-tiled weights on the UMMA M side."""
         b = x.shape[0]
+        if b > 128:  # many rows: the row-major kernel on CTA pairs chooses its own tiles
+            _C.gemm_bf16_tn(w, x, out, True, dual, 1, 0, rows)
+            return
         bn = 16 if b <= 16 else (32 if b <= 32 else (64 if b <= 64 else 128))
         _C.gemm_bf16_tn(w, x, out, True, dual, 1 if b > 64 else splitk, bn, rows)
 
@@ -229,23 +232,43 @@ class TPLlamaDecoder:
         out.copy_(rows * ok[:, None].to(rows.dtype))
 
     def _decode_body(self, B):
-        if self.fused and self.comm.fits_gemm_ar_norm(self.h, B, self.cfg.hidden, self.inter):
+        if self._fused_rows(B):
             return self._decode_body_fused(B)
         return self._decode_body_unfused(B)
+
+    def _fused_rows(self, B):
+        return self.fused and self.comm.fits_gemm_ar_norm(self.h, B, self.cfg.hidden, self.inter)
+
+    def _next_norm(self, li):
+        return self.layers[li + 1]["attn_norm"] if li + 1 < self.cfg.n_layers else self.final_norm
+
+    def _layer_fused(self, li, B, k, v, positions):
+        """One layer for one new token of each of B sequences: xn is normalised again for the next layer."""
+        L, cfg = self.layers[li], self.cfg
+        h, xn, qkv, attn, act = self.h[:B], self.xn[:B], self.qkv[:B], self.attn[:B], self.act[:B]
+        self._gemm_t(L["wqkv"], xn, qkv, self.qkv_rows)
+        _C.decode_attention(qkv, k, v, positions, self.cos, self.sin, attn, self.scratch, self.counters, self.nh, self.nkv, self.nsplit)
+        self.comm.gemm_ar_norm(L["wo"], attn, h, L["mlp_norm"], xn, cfg.eps)
+        self._gemm_t(L["wgu"], xn, act, self.inter, dual=self.inter_pad)
+        self.comm.gemm_ar_norm(L["wd"], act, h, self._next_norm(li), xn, cfg.eps)
+
+    def _layer_unfused(self, li, B, k, v, positions):
+        L, cfg = self.layers[li], self.cfg
+        h, x, xn, qkv, attn, act = self.h[:B], self.x[:B], self.xn[:B], self.qkv[:B], self.attn[:B], self.act[:B]
+        self._gemm_t(L["wqkv"], xn, qkv, self.qkv_rows)
+        _C.decode_attention(qkv, k, v, positions, self.cos, self.sin, attn, self.scratch, self.counters, self.nh, self.nkv, self.nsplit)
+        self._gemm_t(L["wo"], attn, x, cfg.hidden)
+        self.comm.ar_res_norm(x, h, L["mlp_norm"], xn, cfg.eps)
+        self._gemm_t(L["wgu"], xn, act, self.inter, dual=self.inter_pad)
+        self._gemm_t(L["wd"], act, x, cfg.hidden)
+        self.comm.ar_res_norm(x, h, self._next_norm(li), xn, cfg.eps)
 
     def _decode_body_fused(self, B):
         cfg = self.cfg
         tokens, h, xn = self.tokens[:B], self.h[:B], self.xn[:B]
-        qkv, attn, act = self.qkv[:B], self.attn[:B], self.act[:B]
         self.comm.embed_norm(tokens, self.embed, self.rank * self.vshard, h, self.layers[0]["attn_norm"], xn, cfg.eps)
         for li, L in enumerate(self.layers):
-            self._gemm_t(L["wqkv"], xn, qkv, self.qkv_rows)
-            _C.decode_attention(qkv, L["k"], L["v"], self.positions[:B], self.cos, self.sin, attn, self.scratch,
-                                self.counters, self.nh, self.nkv, self.nsplit)
-            self.comm.gemm_ar_norm(L["wo"], attn, h, L["mlp_norm"], xn, cfg.eps)
-            self._gemm_t(L["wgu"], xn, act, self.inter, dual=self.inter_pad)
-            nw = self.layers[li + 1]["attn_norm"] if li + 1 < cfg.n_layers else self.final_norm
-            self.comm.gemm_ar_norm(L["wd"], act, h, nw, xn, cfg.eps)
+            self._layer_fused(li, B, L["k"], L["v"], self.positions[:B])
         self._gemm_t(self.lm_head, xn, self.logits[:B], self.vshard)
         # feeds the sampled ids back into self.tokens and advances the positions: steady state is a pure replay
         self.comm.sample(self.logits[:B], self.next_tokens[:B], tokens, self.positions[:B])
@@ -253,20 +276,11 @@ class TPLlamaDecoder:
     def _decode_body_unfused(self, B):
         cfg = self.cfg
         tokens, h, x, xn = self.tokens[:B], self.h[:B], self.x[:B], self.xn[:B]
-        qkv, attn, act = self.qkv[:B], self.attn[:B], self.act[:B]
         self._embed_partial(tokens, x)
         h.zero_()
         self.comm.ar_res_norm(x, h, self.layers[0]["attn_norm"], xn, cfg.eps)
         for li, L in enumerate(self.layers):
-            self._gemm_t(L["wqkv"], xn, qkv, self.qkv_rows)
-            _C.decode_attention(qkv, L["k"], L["v"], self.positions[:B], self.cos, self.sin, attn, self.scratch,
-                                self.counters, self.nh, self.nkv, self.nsplit)
-            self._gemm_t(L["wo"], attn, x, cfg.hidden)
-            self.comm.ar_res_norm(x, h, L["mlp_norm"], xn, cfg.eps)
-            self._gemm_t(L["wgu"], xn, act, self.inter, dual=self.inter_pad)
-            self._gemm_t(L["wd"], act, x, cfg.hidden)
-            nw = self.layers[li + 1]["attn_norm"] if li + 1 < cfg.n_layers else self.final_norm
-            self.comm.ar_res_norm(x, h, nw, xn, cfg.eps)
+            self._layer_unfused(li, B, L["k"], L["v"], self.positions[:B])
         self._gemm_t(self.lm_head, xn, self.logits[:B], self.vshard)
         val, idx = self.logits[:B].max(dim=-1)
         if self.world > 1:
@@ -325,62 +339,71 @@ class TPLlamaDecoder:
     def prefill(self, prompt, chunk_seqs=None):
         """Runs the prompt [B, S] through the model, fills the KV caches and leaves the first generated
         token in self.tokens. All sequences of a chunk go through every layer together ([chunk * S]
-        rows per GEMM): the same tcgen05 GEMM in its row-major form, the staged all_reduce fused with
-        residual add + norm (in slices that fit the communicator's staging arena), and torch's
-        scaled_dot_product_attention for the causal attention over the prompt itself.
+        rows per GEMM): the tcgen05 GEMM on CTA pairs with the weights as its B operand, one pass for rotary
+        embedding and KV append, torch's scaled_dot_product_attention for the causal attention over the prompt
+        itself (reading K and V where they stay), the all_reduce fused with residual add + norm (in slices that fit
+        the communicator's staging arena). Of the last layer only K and V are wanted for every position; the
+        rest of it runs for the last position of each sequence, as the decode step does.
         `chunk_seqs` bounds the sequences per pass (default: as many as keep a pass under ~32k rows)."""
         cfg = self.cfg
         B, S = prompt.shape
         hd, H = cfg.head_dim, cfg.hidden
         dev = self.device
         bf = dict(device=dev, dtype=torch.bfloat16)
-        cos = self.cos[:S].to(torch.bfloat16)[None, :, None, :]
-        sin = self.sin[:S].to(torch.bfloat16)[None, :, None, :]
-
-        def rope(t):  # [n, S, heads, hd]
-            t1, t2 = t[..., : hd // 2], t[..., hd // 2:]
-            return torch.cat([t1 * cos - t2 * sin, t2 * cos + t1 * sin], dim=-1)
-
+        nq, nkv = self.nh * hd, self.nkv * hd
         cap_rows = 1024 if self.world > 1 else 1 << 30  # rows per fused-norm launch (staging capacity)
         per = chunk_seqs or max(1, 32768 // S)
+        last_li = cfg.n_layers - 1
+        # the packed rows of K and V within wqkv: whole 128-row tiles after those of q
+        kv_off = nq * ((H + 63) // 64)
         for b0 in range(0, B, per):
             n = min(per, B - b0)
             R = n * S
             toks = prompt[b0:b0 + n].reshape(-1).to(dev)
-            x = torch.empty(R, H, **bf)
-            self._embed_partial(toks, x)
-            h = torch.zeros(R, H, **bf)
+            h = torch.empty(R, H, **bf)
             xn = torch.empty(R, H, **bf)
+            if last_li > 0 or self.comm.nccl is not None:
+                x = torch.empty(R, H, **bf)
+                qkv = torch.empty(R, nq + 2 * nkv, **bf)
+                act = torch.empty(R, self.inter, **bf)
 
             def norm_step(w):
                 for r0 in range(0, R, cap_rows):
                     r1 = min(R, r0 + cap_rows)
                     self.comm.ar_res_norm(x[r0:r1], h[r0:r1], w, xn[r0:r1], cfg.eps)
 
-            norm_step(self.layers[0]["attn_norm"])
-            qkv = torch.empty(R, (self.nh + 2 * self.nkv) * hd, **bf)
-            attn = torch.empty(R, self.nh * hd, **bf)
-            act = torch.empty(R, self.inter, **bf)
-            for li, L in enumerate(self.layers):
+            if self.comm.nccl is not None:  # comparison arm: the lookup is reduced by NCCL
+                self._embed_partial(toks, x)
+                h.zero_()
+                norm_step(self.layers[0]["attn_norm"])
+            else:
+                for r0 in range(0, R, cap_rows):
+                    r1 = min(R, r0 + cap_rows)
+                    self.comm.embed_norm(toks[r0:r1], self.embed, self.rank * self.vshard, h[r0:r1], self.layers[0]["attn_norm"],
+                                         xn[r0:r1], cfg.eps)
+            for li, L in enumerate(self.layers[:last_li]):
+                k, v = L["k"][b0:b0 + n], L["v"][b0:b0 + n]
                 self._gemm_t(L["wqkv"], xn, qkv, self.qkv_rows)
-                q = rope(qkv[:, : self.nh * hd].view(n, S, self.nh, hd))
-                k = rope(qkv[:, self.nh * hd:(self.nh + self.nkv) * hd].view(n, S, self.nkv, hd))
-                v = qkv[:, (self.nh + self.nkv) * hd:].view(n, S, self.nkv, hd)
-                L["k"][b0:b0 + n, :, :S] = k.transpose(1, 2)
-                L["v"][b0:b0 + n, :, :S] = v.transpose(1, 2)
+                _C.rope_append(qkv, k, v, self.cos, self.sin, self.nh, S)
                 o = torch.nn.functional.scaled_dot_product_attention(
-                    q.transpose(1, 2), k.transpose(1, 2), v.transpose(1, 2), is_causal=True,
+                    qkv.view(n, S, -1)[..., :nq].view(n, S, self.nh, hd).transpose(1, 2), k[:, :, :S], v[:, :, :S], is_causal=True,
                     enable_gqa=self.nh != self.nkv)
-                attn.copy_(o.transpose(1, 2).reshape(R, self.nh * hd))
-                self._gemm_t(L["wo"], attn, x, cfg.hidden)
+                self._gemm_t(L["wo"], o.transpose(1, 2).reshape(R, nq), x, H)
                 norm_step(L["mlp_norm"])
                 self._gemm_t(L["wgu"], xn, act, self.inter, dual=self.inter_pad)
-                self._gemm_t(L["wd"], act, x, cfg.hidden)
-                nw = self.layers[li + 1]["attn_norm"] if li + 1 < cfg.n_layers else self.final_norm
-                norm_step(nw)
-            last = xn.view(n, S, H)[:, S - 1].contiguous()
+                self._gemm_t(L["wd"], act, x, H)
+                norm_step(self._next_norm(li))
+            L = self.layers[last_li]
+            k, v = L["k"][b0:b0 + n], L["v"][b0:b0 + n]
+            kv = torch.empty(R, 2 * nkv, **bf)
+            self._gemm_t(L["wqkv"][kv_off:], xn, kv, 2 * nkv)
+            _C.rope_append(kv, k, v, self.cos, self.sin, 0, S)
+            self.h[:n].copy_(h.view(n, S, H)[:, S - 1])
+            self.xn[:n].copy_(xn.view(n, S, H)[:, S - 1])
+            (self._layer_fused if self._fused_rows(n) else self._layer_unfused)(
+                last_li, n, k, v, torch.full((n,), S - 1, device=dev, dtype=torch.int32))
             logits = torch.empty(n, self.vshard, device=dev, dtype=torch.float32)
-            self._gemm_t(self.lm_head, last, logits, self.vshard)
+            self._gemm_t(self.lm_head, self.xn[:n], logits, self.vshard)
             val, idx = logits.max(dim=-1)
             if self.world > 1:
                 mine = torch.stack([val, (idx + self.rank * self.vshard).float()], dim=-1).contiguous()
