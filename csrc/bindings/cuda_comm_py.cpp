@@ -56,6 +56,7 @@ void fill_moe_dispatch(ccl::MoeArgs& a, const at::Tensor& x, const at::Tensor& i
   a.topk = (int)idx.size(1);
   a.hidden = (int)x.size(1);
   a.experts_per_rank = experts_per_rank;
+  a.max_rows = (int)out_x.size(0);
 }
 
 void fill_moe_combine(ccl::MoeArgs& a, const at::Tensor& y, const at::Tensor& meta, const at::Tensor& count,

@@ -5,6 +5,7 @@
 
 #include "bindings/common.h"
 #include "cuda/CudaBackend.h"
+#include "cuda/kernels/local_ops.h"
 
 namespace ccl_ops {
 
@@ -88,11 +89,43 @@ void reduce_scatter_cast(ProcessGroupCCL& pg, const at::Tensor& inp, at::Tensor&
     a.scale = (float)scale;
   }
   if (W == 1) {
+    if (at::isFloatingType(inp.scalar_type()) && inp.scalar_type() != at::kDouble) {
+      ccl::CastTable t;
+      t.src[0] = inp.data_ptr();
+      t.off[0] = 0;
+      t.count[0] = (uint64_t)n;
+      t.n = 1;
+      t.dst = out.data_ptr();
+      t.scale = (float)scale;
+      C10_CUDA_CHECK(ccl::launch_cast_table(to_ccl_dtype(inp.scalar_type()), to_ccl_dtype(out.scalar_type()), false, t, c10::cuda::getCurrentCUDAStream()));
+      return;
+    }
     out.copy_(inp.view_as(out));
     if (scale != 1.0) out.mul_(scale);
     return;
   }
   C10_CUDA_CHECK(c.reduce_scatter(to_ccl_dtype(inp.scalar_type()), to_ccl_dtype(out.scalar_type()), {a}, c10::cuda::getCurrentCUDAStream()));
+}
+
+void accumulate_cast(const std::vector<at::Tensor>& src, at::Tensor& dst, const std::vector<int64_t>& offsets, double scale) {
+  TORCH_CHECK(dst.is_cuda() && dst.is_contiguous() && src.size() == offsets.size(), "accumulate_cast: contiguous CUDA destination, one offset per tensor");
+  c10::cuda::CUDAGuard g(dst.device());
+  for (size_t i = 0; i < src.size();) {
+    ccl::CastTable t;
+    t.dst = dst.data_ptr();
+    t.scale = (float)scale;
+    for (; i < src.size() && t.n < ccl::kMaxCastTensors; ++i) {
+      const at::Tensor& s = src[i];
+      same_device(dst, s, "accumulate_cast");
+      TORCH_CHECK(s.is_contiguous() && s.scalar_type() == src[0].scalar_type(), "accumulate_cast: contiguous tensors of one dtype required");
+      TORCH_CHECK(offsets[i] >= 0 && offsets[i] + s.numel() <= dst.numel(), "accumulate_cast: tensor ", i, " does not fit the destination");
+      t.src[t.n] = s.data_ptr();
+      t.off[t.n] = (uint64_t)offsets[i];
+      t.count[t.n] = (uint64_t)s.numel();
+      ++t.n;
+    }
+    C10_CUDA_CHECK(ccl::launch_cast_table(to_ccl_dtype(src[0].scalar_type()), to_ccl_dtype(dst.scalar_type()), true, t, c10::cuda::getCurrentCUDAStream()));
+  }
 }
 
 void all_gather_copy_out(ProcessGroupCCL& pg, const at::Tensor& shard, std::vector<at::Tensor> outs) {
@@ -162,10 +195,14 @@ void all_gather_gemm(ProcessGroupCCL& pg, const at::Tensor& a_shard, const at::T
 }
 
 void moe_dispatch(ProcessGroupCCL& pg, const at::Tensor& x, const at::Tensor& idx, at::Tensor& out_x, at::Tensor& meta,
-                  at::Tensor& count, int64_t experts_per_rank) {
+                  at::Tensor& count, int64_t experts_per_rank, bool clear_count) {
   auto& c = cuda_comm_of(pg, x);
   c10::cuda::CUDAGuard g(x.device());
   ccl::MoeArgs a;
+  if (clear_count) {
+    if (c.world() == 1) a.count_len = (int)count.numel();
+    else count.zero_();
+  }
   ccl_py::fill_moe_dispatch(a, x, idx, out_x, meta, count, (int)experts_per_rank);
   C10_CUDA_CHECK(c.moe_dispatch({a}, c10::cuda::getCurrentCUDAStream()));
 }

@@ -21,11 +21,13 @@ void sample_allgather(ProcessGroupCCL& pg, const at::Tensor& logits, at::Tensor&
                       const c10::optional<at::Tensor>& tokens, const c10::optional<at::Tensor>& positions);
 void all_reduce_scaled(ProcessGroupCCL& pg, at::Tensor& t, double scale);
 void reduce_scatter_cast(ProcessGroupCCL& pg, const at::Tensor& inp, at::Tensor& out, double scale);
+// dst[offsets[i] ...] += scale * src[i] for tensors of one dtype (bf16 / f16 / f32; dst: the same or fp32), in one launch.
+void accumulate_cast(const std::vector<at::Tensor>& src, at::Tensor& dst, const std::vector<int64_t>& offsets, double scale);
 void all_gather_copy_out(ProcessGroupCCL& pg, const at::Tensor& shard, std::vector<at::Tensor> outs);
 void gemm_reduce_scatter(ProcessGroupCCL& pg, const at::Tensor& a, const at::Tensor& b, at::Tensor& out);
 void all_gather_gemm(ProcessGroupCCL& pg, const at::Tensor& a_shard, const at::Tensor& b, at::Tensor& out);
 void moe_dispatch(ProcessGroupCCL& pg, const at::Tensor& x, const at::Tensor& idx, at::Tensor& out_x, at::Tensor& meta,
-                  at::Tensor& count, int64_t experts_per_rank);
+                  at::Tensor& count, int64_t experts_per_rank, bool clear_count = false);  // clear_count: words past 1 + world become 0
 void moe_combine(ProcessGroupCCL& pg, const at::Tensor& y, const at::Tensor& meta, const at::Tensor& count,
                  const at::Tensor& gate, at::Tensor& out);
 

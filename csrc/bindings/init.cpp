@@ -4,6 +4,7 @@
 #include <c10/cuda/CUDAGuard.h>
 
 #include "bindings/common.h"
+#include "bindings/fused_ops.h"
 #include "cuda/kernels/gemm.h"
 
 namespace {
@@ -58,6 +59,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_bf16_tn", &gemm_bf16_tn, py::arg("a"), py::arg("b"), py::arg("out"),
         py::arg("trans_out") = false, py::arg("dual_off") = 0, py::arg("splitk") = 0,
         py::arg("bn") = 0, py::arg("a_tiled_rows") = 0);
+  m.def("accumulate_cast", &ccl_ops::accumulate_cast, py::arg("src"), py::arg("dst"), py::arg("offsets"), py::arg("scale") = 1.0);
   ccl_py::bind_cuda_comm(m);
   ccl_py::bind_process_group(m);
   ccl_py::bind_model_ops(m);

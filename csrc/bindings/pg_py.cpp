@@ -108,7 +108,8 @@ void bind_process_group(py::module& m) {
       .def("fused_gemm_rs", &ccl_ops::gemm_reduce_scatter)
       // out[M, N_local] = all_gather(a_shard)[M, K] @ b[N_local, K]^T
       .def("fused_ag_gemm", &ccl_ops::all_gather_gemm)
-      .def("fused_moe_dispatch", &ccl_ops::moe_dispatch)
+      .def("fused_moe_dispatch", [](ProcessGroupCCL& pg, const at::Tensor& x, const at::Tensor& idx, at::Tensor& out_x, at::Tensor& meta,
+                                    at::Tensor& count, int64_t experts_per_rank) { ccl_ops::moe_dispatch(pg, x, idx, out_x, meta, count, experts_per_rank); })
       .def("fused_moe_combine", &ccl_ops::moe_combine)
       // staging capacity (bytes) of the fused GEMM + collective ops: the whole M x N (gemm_rs) or M x K (ag_gemm) bf16 matrix must fit
       .def("fused_gemm_capacity_bytes", [](ProcessGroupCCL& pg, const at::Tensor& like) { return (int64_t)cuda_comm_of(pg, like).config().half_bytes; })

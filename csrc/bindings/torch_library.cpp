@@ -71,8 +71,8 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor> moe_dispatch_cuda(const at::Tenso
                                                                  int64_t experts_per_rank, int64_t max_rows, const std::string& group) {
   at::Tensor out_x = at::empty({max_rows, x.size(1)}, x.options());
   at::Tensor meta = at::empty({max_rows, 3}, x.options().dtype(at::kInt));
-  at::Tensor count = at::zeros({16}, x.options().dtype(at::kInt));
-  ccl_ops::moe_dispatch(backend_of(group, x), x, expert_idx, out_x, meta, count, experts_per_rank);
+  at::Tensor count = at::empty({16}, x.options().dtype(at::kInt));
+  ccl_ops::moe_dispatch(backend_of(group, x), x, expert_idx, out_x, meta, count, experts_per_rank, /*clear_count=*/true);
   return {out_x, meta, count};
 }
 at::Tensor moe_combine_cuda(const at::Tensor& y, const at::Tensor& meta, const at::Tensor& count, const at::Tensor& gate,

@@ -18,6 +18,8 @@
 #include "comm.cuh"
 #include "gemm.h"
 
+#include <algorithm>
+
 namespace ccl {
 namespace {
 
@@ -215,6 +217,126 @@ __global__ void __launch_bounds__(512) moe_combine_kernel(const __grid_constant_
   sy.finish(1);
 }
 
+// ---------------------------------------------------------------------------------------------
+// One-rank communicators: nothing crosses a link, so nothing is staged. Dispatch reads a token once and writes its topk
+// rows in (token, k) order; combine gathers the rows of a token through the inverse of `meta` (a program may have
+// reordered rows and meta together, by expert for example) and writes the sum. Bound by memory: (1 + topk) rows read
+// and written per token in each direction. A thread moves two vectors per row, a CTA one token, so that the whole chip
+// has loads in flight: the staged kernels move every row twice with 64 CTAs and wait for one another in between
+// (4096 tokens x 4096, top 2: 150 us to dispatch, 160 us to combine).
+// ---------------------------------------------------------------------------------------------
+__global__ void __launch_bounds__(256) moe_dispatch_local_kernel(const MoeArgs a, int* status) {
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
+  const int t = blockIdx.x;
+  const int hv = a.hidden / 8;
+  const int limit = min(a.cap, a.max_rows);
+  if (blockIdx.y == 0) {
+    for (int k = threadIdx.x; k < a.topk && t < a.tokens; k += blockDim.x) {
+      const int r = t * a.topk + k;
+      if (r < limit) {
+        a.out_meta[3 * r] = 0;
+        a.out_meta[3 * r + 1] = r;
+        a.out_meta[3 * r + 2] = a.expert_idx[r];
+      } else if (status) {
+        atomicCAS(status, kStatusOk, kStatusBounds);  // over capacity: the row is dropped and the error recorded
+      }
+    }
+    if (t == 0) {  // (also the only CTA of a call without tokens)
+      const int n = max(a.count_len, 2);
+      for (int i = threadIdx.x; i < n; i += blockDim.x) a.out_count[i] = i < 2 ? min(a.tokens * a.topk, limit) : 0;
+    }
+  }
+  if (t >= a.tokens) return;
+  const uint4* src = reinterpret_cast<const uint4*>(a.x) + (size_t)t * hv;
+  const int i0 = blockIdx.y * 2 * blockDim.x + threadIdx.x, i1 = i0 + blockDim.x;
+  uint4 v0 = make_uint4(0, 0, 0, 0), v1 = v0;
+  if (i0 < hv) v0 = ptx::ld_nc_v4(src + i0);
+  if (i1 < hv) v1 = ptx::ld_nc_v4(src + i1);
+  for (int k = 0; k < a.topk; ++k) {
+    const int r = t * a.topk + k;
+    if (r >= limit) break;
+    uint4* dst = reinterpret_cast<uint4*>(a.out_x) + (size_t)r * hv;
+    if (i0 < hv) dst[i0] = v0;
+    if (i1 < hv) dst[i1] = v1;
+  }
+}
+
+__global__ void __launch_bounds__(256) moe_inverse_kernel(const MoeArgs a, int* inverse) {
+  ptx::griddep_launch_dependents();
+  ptx::griddep_wait();
+  const int rows = a.in_rows[0];
+  const int slots = a.tokens * a.topk;
+  for (int r = blockIdx.x * blockDim.x + threadIdx.x; r < rows; r += gridDim.x * blockDim.x) {
+    const int slot = a.out_meta[3 * r + 1];
+    if (slot >= 0 && slot < slots) inverse[slot] = r;
+  }
+}
+
+constexpr int kCombineBatch = 4;  // rows of a token in flight at once
+
+__global__ void __launch_bounds__(256) moe_combine_local_kernel(const MoeArgs a, const int* inverse) {
+  ptx::griddep_launch_dependents();
+  const int t = blockIdx.x;
+  const int hv = a.hidden / 8;
+  ptx::griddep_wait();
+  const int rows = a.in_rows[0];
+  const int i0 = blockIdx.y * 2 * blockDim.x + threadIdx.x;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int i = i0 + h * blockDim.x;
+    if (i >= hv) break;
+    float acc[8];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) acc[q] = 0.f;
+    for (int k0 = 0; k0 < a.topk; k0 += kCombineBatch) {
+      Vec<__nv_bfloat16> v[kCombineBatch];
+      float w[kCombineBatch];
+#pragma unroll
+      for (int k = 0; k < kCombineBatch; ++k) {
+        w[k] = 0.f;
+        if (k0 + k < a.topk) {
+          const int slot = t * a.topk + k0 + k;
+          const int r = inverse[slot];
+          const bool ok = r >= 0 && r < rows;  // a slot that no row came back for counts as zero
+          *reinterpret_cast<uint4*>(&v[k]) = ok ? ptx::ld_nc_v4(reinterpret_cast<const uint4*>(a.x) + (size_t)r * hv + i) : make_uint4(0, 0, 0, 0);
+          w[k] = a.gate[slot];
+        }
+      }
+#pragma unroll
+      for (int k = 0; k < kCombineBatch; ++k) {
+        if (k0 + k < a.topk) {
+#pragma unroll
+          for (int q = 0; q < 8; ++q) acc[q] += w[k] * __bfloat162float(v[k].v[q]);
+        }
+      }
+    }
+    Vec<__nv_bfloat16> o;
+#pragma unroll
+    for (int q = 0; q < 8; ++q) o.v[q] = __float2bfloat16(acc[q]);
+    reinterpret_cast<uint4*>(a.out_x)[(size_t)t * hv + i] = *reinterpret_cast<const uint4*>(&o);
+  }
+}
+
+template <typename K, typename... Args>
+cudaError_t launch_local(K kern, dim3 grid, int threads, cudaStream_t stream, const Args&... args) {
+  cudaLaunchConfig_t lc = {};
+  lc.gridDim = grid;
+  lc.blockDim = dim3(threads);
+  lc.stream = stream;
+  cudaLaunchAttribute attr[1];
+  lc.attrs = attr;
+  lc.numAttrs = pdl_launch_attr(&attr[0]);
+  return cudaLaunchKernelEx(&lc, kern, args...);
+}
+
+// Threads of a CTA that moves one token (two vectors each), and how many CTAs share a long row.
+dim3 local_grid(const MoeArgs& a, int* threads) {
+  const int hv = a.hidden / 8;
+  *threads = hv >= 512 ? 256 : ((hv + 1) / 2 + 31) / 32 * 32;
+  return dim3(std::max(a.tokens, 1), (hv + 2 * *threads - 1) / (2 * *threads), 1);
+}
+
 template <typename KR, typename KE>
 cudaError_t launch_moe(KR kreal, KE kemu, const RankCtx* ctx, const MoeArgs* args, const LaunchCfg& cfg) {
   dim3 block(cfg.nthreads);
@@ -250,9 +372,26 @@ size_t moe_dispatch_slot_bytes(int cap, int hidden) {
 }
 
 cudaError_t launch_moe_dispatch(const RankCtx* ctx, const MoeArgs* args, const LaunchCfg& cfg) {
+  if (!cfg.cooperative && ctx->world == 1) {
+    int threads = 0;
+    const dim3 grid = local_grid(*args, &threads);
+    return launch_local(moe_dispatch_local_kernel, grid, threads, cfg.stream, *args, ctx->status);
+  }
   return launch_moe(moe_dispatch_kernel<false>, moe_dispatch_kernel<true>, ctx, args, cfg);
 }
 cudaError_t launch_moe_combine(const RankCtx* ctx, const MoeArgs* args, const LaunchCfg& cfg) {
+  if (!cfg.cooperative && ctx->world == 1) {
+    // the inverse (a word per slot) lives in the arena, which nothing else of a one-rank communicator uses
+    int* inverse = reinterpret_cast<int*>(ctx->data[0]);
+    const int slots = args->tokens * args->topk;
+    if (args->tokens == 0) return cudaSuccess;
+    if ((size_t)slots * sizeof(int) > ctx->half_bytes) return cudaErrorInvalidValue;
+    cudaError_t e = launch_local(moe_inverse_kernel, dim3(std::min((slots + 255) / 256, 592)), 256, cfg.stream, *args, inverse);
+    if (e != cudaSuccess) return e;
+    int threads = 0;
+    const dim3 grid = local_grid(*args, &threads);
+    return launch_local(moe_combine_local_kernel, grid, threads, cfg.stream, *args, static_cast<const int*>(inverse));
+  }
   return launch_moe(moe_combine_kernel<false>, moe_combine_kernel<true>, ctx, args, cfg);
 }
 

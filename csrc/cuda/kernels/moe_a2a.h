@@ -21,6 +21,8 @@ struct MoeArgs {
   int experts_per_rank = 1;
   int cap = 0;                      // rows one source may send to one destination
   unsigned long long slot_bytes = 0;  // moe_dispatch_slot_bytes(cap, hidden)
+  int max_rows = 0;                 // dispatch: rows that out_x holds
+  int count_len = 0;                // dispatch: words of out_count to define (0: only those listed above)
 };
 
 size_t moe_dispatch_slot_bytes(int cap, int hidden);

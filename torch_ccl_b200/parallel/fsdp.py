@@ -10,6 +10,9 @@ parameter, an fp32 master copy of that shard and an fp32 gradient shard. Around 
     them over the ranks, averages, and writes fp32 into the gradient shard in the same kernel
     (`ops.reduce_scatter_cast`: no separate divide and no separate cast).
 
+With one rank there is nothing to gather or to scatter: the parameters are views of the shard itself, and the
+gradients that autograd produced are added to the fp32 gradient shard in one launch, straight from where they are.
+
 Activations inside a unit are recomputed in backward (the unit runs under no_grad in forward), so
 only unit boundaries are kept. The all_gather of the next unit (previous unit in backward) is
 prefetched on a side stream while the current unit computes.
@@ -25,7 +28,7 @@ backend. This engine exists to exercise the fused reduce_scatter / all_gather ke
 import torch
 import torch.distributed as dist
 
-from .. import ops
+from .. import _C, ops
 
 
 class _SymmPool:
@@ -69,7 +72,8 @@ class ShardedUnit:
         self.shard = flat[lo:lo + self.shard_numel].clone()
         self.master = self.shard.float()               # fp32 master weights of the shard
         self.grad_shard = torch.zeros_like(self.master)  # fp32 gradient of the shard
-        self._rs_out = torch.empty_like(self.master)
+        self.alone = self.world == 1 and comm == "ccl"
+        self._rs_out = None if self.alone else torch.empty_like(self.master)
         del flat
         for p in self.params:
             p.data = torch.empty(0, device=dev, dtype=param_dtype)
@@ -83,6 +87,11 @@ class ShardedUnit:
     def gather(self, stream):
         """All-gather the flat parameter; parameters become views of the gathered buffer."""
         if self.full is not None:
+            return
+        if self.alone:
+            self.full = self.shard
+            for p, (o, n, shape) in zip(self.params, self.meta):
+                p.data = self.shard[o:o + n].view(shape)
             return
         cur = torch.cuda.current_stream(self.device)
         s = stream
@@ -121,6 +130,10 @@ class ShardedUnit:
 
     # -- gradients ----------------------------------------------------------------------------
     def prepare_grads(self):
+        if self.alone:
+            for p in self.params:
+                p.grad = None  # autograd hands its own tensors over
+            return
         if self.gpool is not None:
             if self.gpool.free[self.slot] is not None:
                 torch.cuda.current_stream(self.device).wait_event(self.gpool.free[self.slot])  # its last reduce_scatter is done
@@ -137,6 +150,14 @@ class ShardedUnit:
         Runs on `stream` — the same stream as the parameter gathers: the kernels of one
         communicator must never run concurrently, so all of the engine's collectives share one
         stream and are ordered against the compute stream with events."""
+        if self.alone:
+            # on the compute stream: the gradients are freed in its order, and the pass is 10 bytes per parameter
+            got = [(p.grad.contiguous(), o) for p, (o, _, _) in zip(self.params, self.meta) if p.grad is not None]
+            if got:
+                _C.accumulate_cast([g for g, _ in got], self.grad_shard, [o for _, o in got], 1.0)
+            for p in self.params:
+                p.grad = None
+            return
         cur = torch.cuda.current_stream(self.device)
         done = torch.cuda.Event()
         done.record(cur)
