@@ -1,5 +1,6 @@
 #include "cuda/CudaComm.h"
 #include "cuda/Tuner.h"
+#include "cuda/kernels/gemm.h"
 
 #include <algorithm>
 #include <chrono>
@@ -536,10 +537,33 @@ cudaError_t CudaComm::barrier(cudaStream_t stream) {
   return e;
 }
 
+cudaError_t CudaComm::plain_gemm(const void* a, const void* b, void* out, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb,
+                                 int64_t ldo, cudaStream_t stream) {
+  GemmDesc d;
+  d.a = a;
+  d.b = b;
+  d.out = out;
+  d.M = M;
+  d.N = N;
+  d.K = K;
+  d.lda = lda;
+  d.ldb = ldb;
+  d.ldo = ldo;
+  cudaError_t e = gemm_bf16_tn(d, stream);
+  if (e == cudaSuccess) ++launches_;
+  return e;
+}
+
 cudaError_t CudaComm::gemm_rs(const std::vector<GemmRsArgs>& args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
   enter_stream(stream);
+  if (world_ == 1) {
+    // nobody to exchange with: the plain kernel straight into the result (no staging, no reduce pass)
+    const GemmRsArgs& a = args[0];
+    if (a.M % 128 != 0 || a.N % 16 != 0 || a.K % 8 != 0) return cudaErrorInvalidValue;
+    return plain_gemm(a.a, a.b, a.out, a.M, a.N, a.K, a.lda, a.ldb, a.N, stream);
+  }
   // every rank's GEMM only pushes and signals; the reduce kernels wait. Played one rank after
   // the other in emulation, which is safe because the pushes never wait.
   for (int i = 0; i < nctx(); ++i) {
@@ -561,6 +585,11 @@ cudaError_t CudaComm::ag_gemm(const std::vector<AgGemmArgs>& args, cudaStream_t 
   DeviceGuard g(device_);
   enter_stream(stream);
   const int ncomm = 8;
+  if (world_ == 1) {
+    const AgGemmArgs& a = args[0];
+    if (a.M % 128 != 0 || a.K % 8 != 0 || a.lda != a.K) return cudaErrorInvalidValue;
+    return plain_gemm(a.a_shard, a.b, a.out, a.M, a.N, a.K, a.lda, a.ldb, a.ldo, stream);
+  }
   if (!emulated_) {
     cudaError_t e = launch_ag_gemm(host_ctx_[0], args[0], 0, ncomm, stream);
     if (e == cudaSuccess) ++launches_;

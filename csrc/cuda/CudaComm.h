@@ -180,6 +180,8 @@ class CudaComm {
 
  private:
   void init_tables();
+  cudaError_t plain_gemm(const void* a, const void* b, void* out, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldo,
+                         cudaStream_t stream);
   void enter_stream(cudaStream_t s);
   template <typename ArgsT>
   const ArgsT* upload(const std::vector<ArgsT>& args, cudaStream_t stream);

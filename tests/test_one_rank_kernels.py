@@ -1,0 +1,129 @@
+"""Kernels that only a one-rank communicator takes (nothing to exchange, so nothing is staged), and the prompt-side
+kernel, against plain PyTorch, at the edges of their grids."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def comm():
+    import torch_ccl_b200._C as C
+
+    return C.CudaComm.create(None, 0, 1, 8 << 20, 1000, "ccl/one-rank-test")
+
+
+# one row / the last row count of the wide form and the first of the narrow one / hidden from one vector to the largest
+@pytest.mark.parametrize("rows,hidden", [(1, 8), (3, 4096), (592, 952), (593, 952), (700, 4096), (5, 5120), (600, 16384)])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_residual_rmsnorm(comm, rows, hidden, dtype):
+    g = torch.Generator(device="cuda").manual_seed(rows * hidden)
+    x, res, w = (torch.randn(*s, generator=g, device="cuda").to(dtype) for s in ((rows, hidden), (rows, hidden), (hidden,)))
+    h = (x.float() + res.float()).to(dtype)
+    n = (h.float() * torch.rsqrt(h.float().pow(2).mean(-1, keepdim=True) + 1e-5)).to(dtype)
+    out = torch.empty_like(x)
+    comm.allreduce_residual_rmsnorm([x], [res], [w], [out], 1e-5)
+    assert torch.equal(res, h)
+    # half a unit in the last place is at most 2^-8 (bf16: 8 significant bits) or 2^-11 (f16: 11 bits) of a value. The mean
+    # in another order may move the normalised value by one unit in the last place (two halves), and the product with the
+    # weight is rounded (one half): three halves in all.
+    half = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-11
+    torch.testing.assert_close(out.float(), n.float() * w.float(), rtol=3 * half, atol=1e-6)
+
+
+def test_residual_rmsnorm_embedding(comm):
+    """Token ids outside this rank's part of the table contribute zeros; the residual is not read."""
+    table = torch.randn(50, 256, device="cuda").bfloat16()
+    tok = torch.tensor([0, 99, 100, 149, 150, 7], device="cuda")
+    res = torch.full((6, 256), float("nan"), device="cuda", dtype=torch.bfloat16)
+    out = torch.empty_like(res)
+    comm.allreduce_residual_rmsnorm([table], [res], [torch.ones(256, device="cuda").bfloat16()], [out], 1e-5, [tok], [100], True)
+    want = torch.zeros_like(res)
+    want[2], want[3] = table[0], table[49]
+    assert torch.equal(res, want) and not torch.isnan(out.float()).any()
+
+
+@pytest.mark.parametrize("n,seq,heads,kv,room", [(1, 1, 4, 4, 8), (3, 77, 8, 2, 80), (2, 130, 0, 3, 130)])
+def test_rope_append(n, seq, heads, kv, room):
+    import torch_ccl_b200._C as C
+
+    g = torch.Generator(device="cuda").manual_seed(seq)
+    qkv = torch.randn(n * seq, (heads + 2 * kv) * 128, generator=g, device="cuda").bfloat16()
+    inv = 1.0 / (10000.0 ** (torch.arange(0, 128, 2, device="cuda").float() / 128))
+    ang = torch.arange(room, device="cuda").float()[:, None] * inv[None]
+    cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+    c, s = (t[:seq].bfloat16()[None, :, None] for t in (cos, sin))
+    x = qkv.view(n, seq, -1, 128).clone()
+    t1, t2 = x[:, :, : heads + kv, :64], x[:, :, : heads + kv, 64:]
+    rot = torch.cat([t1 * c - t2 * s, t2 * c + t1 * s], -1)
+    kc = torch.full((n, kv, room, 128), 7.0, device="cuda", dtype=torch.bfloat16)
+    vc = kc.clone()
+    C.rope_append(qkv, kc, vc, cos, sin, heads, seq)
+    got = qkv.view(n, seq, -1, 128)
+    assert torch.equal(got[:, :, :heads], rot[:, :, :heads]) and torch.equal(got[:, :, heads:], x[:, :, heads:])
+    assert torch.equal(kc[:, :, :seq], rot[:, :, heads:].transpose(1, 2)) and torch.equal(vc[:, :, :seq], x[:, :, heads + kv:].transpose(1, 2))
+    assert (kc[:, :, seq:] == 7.0).all() and (vc[:, :, seq:] == 7.0).all()
+
+
+@pytest.mark.parametrize("tokens,hidden,experts,topk", [(0, 64, 2, 1), (1, 8, 4, 1), (33, 256, 8, 2), (100, 4104, 16, 5), (7, 8192, 8, 9)])
+def test_moe(comm, tokens, hidden, experts, topk):
+    """Dispatch in slot order; combine from any order of rows and records; a slot whose row is missing counts as zero."""
+    g = torch.Generator(device="cuda").manual_seed(hidden)
+    x = torch.randn(tokens, hidden, generator=g, device="cuda").bfloat16()
+    idx = torch.randint(0, experts, (tokens, topk), generator=g, device="cuda", dtype=torch.int32)
+    gate = torch.rand(tokens, topk, generator=g, device="cuda")
+    n = tokens * topk
+    rows = torch.empty(n, hidden, device="cuda", dtype=torch.bfloat16)
+    meta = torch.empty(n, 3, device="cuda", dtype=torch.int32)
+    count = torch.full((16,), -1, device="cuda", dtype=torch.int32)
+    comm.moe_dispatch([x], [idx], [rows], [meta], [count], experts)
+    assert count[:2].tolist() == [n, n] and (count[2:] == -1).all()
+    assert torch.equal(rows, x.repeat_interleave(topk, 0)) and torch.equal(meta[:, 2], idx.view(-1)) and comm.status()[0] == 0
+    y = (rows.float() * (1 + meta[:, 2:3])).bfloat16()
+    p = torch.randperm(n, device="cuda")
+    out = torch.empty(tokens, hidden, device="cuda", dtype=torch.bfloat16)
+    comm.moe_combine([y[p].contiguous()], [meta[p].contiguous()], [count], [gate], [out])
+    ref = (y.double().view(tokens, topk, hidden) * gate.double()[:, :, None]).sum(1)
+    # fp32 sum of topk products (2^-24 each of their magnitude), then one rounding to bf16
+    bound = ref.abs() * 2.0**-8 + (y.double().view(tokens, topk, hidden).abs() * gate.double()[:, :, None]).sum(1) * topk * 2.0**-23
+    assert ((out.double() - ref).abs() <= bound).all()
+
+
+def test_moe_over_capacity(comm):
+    """Rows that out_x has no room for are dropped and reported."""
+    x, idx = torch.ones(4, 64, device="cuda").bfloat16(), torch.zeros(4, 2, device="cuda", dtype=torch.int32)
+    store = torch.full((8, 64), 5.0, device="cuda").bfloat16()
+    meta, count = torch.zeros(8, 3, device="cuda", dtype=torch.int32), torch.zeros(16, device="cuda", dtype=torch.int32)
+    comm.moe_dispatch([x], [idx], [store[:6]], [meta], [count], 1)
+    torch.cuda.synchronize()
+    assert comm.status()[0] == 2 and int(count[0]) == 6 and (store[6:] == 5.0).all()
+    comm.clear_status()
+
+
+@pytest.mark.parametrize("sizes", [[1], [7, 8, 9], [4096, 3, 100001], [5] * 60])
+@pytest.mark.parametrize("src,dst", [(torch.bfloat16, torch.float32), (torch.float16, torch.float32), (torch.float32, torch.float32),
+                                     (torch.bfloat16, torch.bfloat16)])
+def test_accumulate_cast(sizes, src, dst):
+    """Any offsets (so any alignment of the destination), more tensors than one launch takes."""
+    import torch_ccl_b200._C as C
+
+    g = torch.Generator(device="cuda").manual_seed(len(sizes))
+    xs = [torch.randn(n, generator=g, device="cuda").to(src) for n in sizes]
+    offs = [sum(sizes[:i]) + 3 for i in range(len(sizes))]
+    acc = torch.randn(sum(sizes) + 8, generator=g, device="cuda").to(dst)
+    want = acc.clone()
+    for x, o in zip(xs, offs):
+        want[o:o + x.numel()] = (want[o:o + x.numel()].float() + x.float() * 0.5).to(dst)
+    C.accumulate_cast(xs, acc, offs, 0.5)
+    assert torch.equal(acc, want)  # the product with 0.5 is exact, so a fused multiply-add rounds the same
+
+
+@pytest.mark.parametrize("M,N,K", [(128, 16, 64), (384, 1024, 520)])
+def test_gemm_collective_ops_alone(comm, M, N, K):
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, b = torch.randn(M, K, generator=g, device="cuda").bfloat16(), torch.randn(N, K, generator=g, device="cuda").bfloat16()
+    ref = a.float() @ b.float().t()
+    for op in (comm.gemm_rs, comm.ag_gemm):
+        out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
+        op([a], [b], [out])
+        assert ((out.float() - ref).norm() / ref.norm()).item() <= 2.0**-9 + K * 2.0**-24

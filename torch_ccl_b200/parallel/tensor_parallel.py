@@ -29,6 +29,8 @@ def _world(group):
 
 
 def _all_gather_rows(x, group):
+    if _world(group) == 1:
+        return x
     out = torch.empty((x.shape[0] * _world(group),) + tuple(x.shape[1:]), device=x.device, dtype=x.dtype)
     dist.all_gather_into_tensor(out, x.contiguous(), group=group)
     return out
@@ -36,6 +38,8 @@ def _all_gather_rows(x, group):
 
 def _reduce_scatter_rows(x, group):
     w = _world(group)
+    if w == 1:
+        return x
     out = torch.empty((x.shape[0] // w,) + tuple(x.shape[1:]), device=x.device, dtype=x.dtype)
     dist.reduce_scatter_tensor(out, x.contiguous(), group=group)
     return out
