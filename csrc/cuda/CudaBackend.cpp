@@ -118,7 +118,7 @@ class CudaWork : public AsyncWork {
     if (!stream_ || stream_->stream() != cur) C10_CUDA_CHECK(cudaStreamWaitEvent(cur, end_->ev, 0));
     // From here on the issuing stream runs after the kernels, so the tensors may be freed in its order. (Waiting on
     // another stream says nothing about the one they were allocated for: the watchdog keeps them then.)
-    if (keep_ && cur == issued_from_) keep_->drop();
+    if (keep_ && cur == issued_from_) keep_->drop_after(c10::cuda::getCurrentCUDAStream(device_.index()));
   }
 
   int cudaDevice() const override { return device_.index(); }
@@ -163,6 +163,26 @@ Watchdog& Watchdog::get() {
 }
 
 Watchdog::Watchdog() : th_([this] { loop(); }) {}
+
+// Memory of torch's caching allocator: freed in stream order, and told about other streams that use it (which costs nothing
+// for the stream it was allocated on). Anything else, such as the symmetric heap, is free for its next user at once.
+static bool stream_ordered(const at::Tensor& t) {
+  return t.storage().data_ptr().get_deleter() == c10::cuda::CUDACachingAllocator::get()->raw_deleter();
+}
+
+void Watchdog::KeepAlive::drop_after(c10::cuda::CUDAStream stream) {
+  std::vector<at::Tensor> gone, rest;  // freed outside the lock
+  std::lock_guard<std::mutex> g(mu);
+  for (auto& t : tensors) {
+    if (!stream_ordered(t)) {
+      rest.push_back(std::move(t));
+      continue;
+    }
+    c10::cuda::CUDACachingAllocator::recordStream(t.storage().data_ptr(), stream);
+    gone.push_back(std::move(t));
+  }
+  tensors.swap(rest);
+}
 
 void Watchdog::enqueue(Item item) {
   bool wake;
@@ -521,12 +541,11 @@ c10::intrusive_ptr<c10d::Work> CudaBackendImpl::run(c10d::OpType type, const cha
   item.work = c10::weak_intrusive_ptr<AsyncWork>(work);
   item.end = work->end_;
   item.comm = comm_;
-  if (fork) {
-    // keeps the tensors alive while another stream uses them (instead of record_stream)
-    item.keep = std::make_shared<Watchdog::KeepAlive>();
-    item.keep->tensors = keep;
-    work->keep_ = item.keep;
-  }
+  // keeps the tensors alive while another stream uses them (instead of record_stream)
+  item.keep = std::make_shared<Watchdog::KeepAlive>();
+  item.keep->tensors = keep;
+  if (fork) work->keep_ = item.keep;
+  else item.keep->drop_after(stream);
   item.stream = stream.stream();
   item.flight_slot = work->flight_slot;
   item.seq = seq;

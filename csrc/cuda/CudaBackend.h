@@ -98,6 +98,8 @@ class Watchdog {
       std::lock_guard<std::mutex> g(mu);
       gone.swap(tensors);
     }
+    // `stream` runs after the kernels: gives the tensors up in its order, whichever stream they were allocated for.
+    void drop_after(c10::cuda::CUDAStream stream);
   };
   struct Item {
     c10::weak_intrusive_ptr<c10d::ProcessGroupCCL::AsyncWorkCCL> work;

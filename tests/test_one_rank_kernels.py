@@ -127,3 +127,44 @@ def test_gemm_collective_ops_alone(comm, M, N, K):
         out = torch.empty(M, N, device="cuda", dtype=torch.bfloat16)
         op([a], [b], [out])
         assert ((out.float() - ref).norm() / ref.norm()).item() <= 2.0**-9 + K * 2.0**-24
+
+
+@pytest.fixture()
+def group():
+    import torch.distributed as dist
+
+    import oneccl_bindings_for_pytorch  # noqa: F401
+
+    dist.init_process_group("ccl", store=dist.HashStore(), rank=0, world_size=1)
+    yield dist.group.WORLD
+    dist.destroy_process_group()
+
+
+@pytest.mark.parametrize("async_op", [False, True])
+def test_tensor_of_another_stream_outlives_the_collective(group, async_op):
+    """A tensor allocated on one stream, used by a collective issued from another and freed at once: its memory is not
+    handed out on the first stream while the collective is pending."""
+    import torch.distributed as dist
+
+    n = 1 << 20
+    home = torch.cuda.Stream()
+    with torch.cuda.stream(home):
+        t = torch.ones(n, device="cuda")
+    torch.cuda.current_stream().wait_stream(home)
+    out = torch.empty(n, device="cuda")
+    # set-up of the communicator, and everything loaded: loading a kernel may wait for the device
+    dist.all_gather_into_tensor(out, torch.zeros(n, device="cuda"), group=group, async_op=async_op)
+    torch.cuda._sleep(1000)
+    torch.cuda.synchronize()
+    torch.cuda._sleep(200_000_000)  # about 0.1 s of device time before the collective may run
+    work = dist.all_gather_into_tensor(out, t, group=group, async_op=async_op)
+    if async_op:
+        work.wait()
+        del work
+    was = t.data_ptr()
+    del t
+    with torch.cuda.stream(home):
+        other = torch.zeros(n, device="cuda")
+    assert other.data_ptr() != was
+    torch.cuda.synchronize()
+    assert (out == 1).all()
