@@ -298,7 +298,8 @@ __global__ void __launch_bounds__(256) moe_combine_local_kernel(const MoeArgs a,
         if (k0 + k < a.topk) {
           const int slot = t * a.topk + k0 + k;
           const int r = inverse[slot];
-          const bool ok = r >= 0 && r < rows;  // a slot that no row came back for counts as zero
+          // a slot that no row came back for counts as zero: its word of the inverse may be one of an earlier call
+          const bool ok = r >= 0 && r < rows && a.out_meta[3 * r + 1] == slot;
           *reinterpret_cast<uint4*>(&v[k]) = ok ? ptx::ld_nc_v4(reinterpret_cast<const uint4*>(a.x) + (size_t)r * hv + i) : make_uint4(0, 0, 0, 0);
           w[k] = a.gate[slot];
         }

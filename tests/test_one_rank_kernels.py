@@ -87,6 +87,13 @@ def test_moe(comm, tokens, hidden, experts, topk):
     # fp32 sum of topk products (2^-24 each of their magnitude), then one rounding to bf16
     bound = ref.abs() * 2.0**-8 + (y.double().view(tokens, topk, hidden).abs() * gate.double()[:, :, None]).sum(1) * topk * 2.0**-23
     assert ((out.double() - ref).abs() <= bound).all()
+    if n:  # the last row does not come back
+        count[0] = n - 1
+        comm.moe_combine([y[p].contiguous()], [meta[p].contiguous()], [count], [gate], [out])
+        left = y.clone()
+        left[int(meta[p[-1], 1])] = 0
+        ref = (left.double().view(tokens, topk, hidden) * gate.double()[:, :, None]).sum(1)
+        assert ((out.double() - ref).abs() <= bound + ref.abs() * 2.0**-8).all()
 
 
 def test_moe_over_capacity(comm):
