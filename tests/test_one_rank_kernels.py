@@ -175,3 +175,17 @@ def test_tensor_of_another_stream_outlives_the_collective(group, async_op):
     assert other.data_ptr() != was
     torch.cuda.synchronize()
     assert (out == 1).all()
+
+
+def test_full_shard_unit_with_a_sparse_gradient(group):
+    from torch_ccl_b200.parallel.fsdp import FullyShardedSequential
+
+    torch.manual_seed(0)
+    emb = torch.nn.Embedding(40, 16, sparse=True, device="cuda")
+    engine = FullyShardedSequential([emb], group=group)
+    ids = torch.tensor([[3, 5, 3]], device="cuda")
+    engine(ids).backward(torch.ones(1, 3, 16, device="cuda", dtype=torch.bfloat16))
+    grad = engine.master_params()[0].grad[: 40 * 16].view(40, 16)
+    want = torch.zeros(40, 16, device="cuda")
+    want[3], want[5] = 2.0, 1.0
+    assert torch.equal(grad, want)

@@ -72,7 +72,7 @@ class ShardedUnit:
         self.shard = flat[lo:lo + self.shard_numel].clone()
         self.master = self.shard.float()               # fp32 master weights of the shard
         self.grad_shard = torch.zeros_like(self.master)  # fp32 gradient of the shard
-        self.alone = self.world == 1 and comm == "ccl"
+        self.alone = self.world == 1 and comm == "ccl" and param_dtype in (torch.bfloat16, torch.float16, torch.float32)
         self._rs_out = None if self.alone else torch.empty_like(self.master)
         del flat
         for p in self.params:
@@ -152,7 +152,8 @@ class ShardedUnit:
         stream and are ordered against the compute stream with events."""
         if self.alone:
             # on the compute stream: the gradients are freed in its order, and the pass is 10 bytes per parameter
-            got = [(p.grad.contiguous(), o) for p, (o, _, _) in zip(self.params, self.meta) if p.grad is not None]
+            got = [((p.grad.to_dense() if p.grad.is_sparse else p.grad).contiguous(), o)
+                   for p, (o, _, _) in zip(self.params, self.meta) if p.grad is not None]
             if got:
                 _C.accumulate_cast([g for g, _ in got], self.grad_shard, [o for _, o in got], 1.0)
             for p in self.params:
