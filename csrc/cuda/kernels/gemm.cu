@@ -193,7 +193,6 @@ cudaError_t launch(const GemmDesc& d, int splitk, cudaStream_t stream) {
   CUtensorMap ta, tb;
   const int64_t a_rows = DUAL ? (d.dual_off + d.M) : d.M;
   if (d.a_tiled) {
-    if (d.dual_off % kBM != 0) return cudaErrorInvalidValue;
     if (!tma::make_2d_bf16(&ta, d.a, (uint64_t)d.a_packed_rows, (uint64_t)kBK, (uint64_t)kBK, kBM, kBK))
       return cudaErrorInvalidValue;
   } else if (!tma::make_2d_bf16(&ta, d.a, (uint64_t)a_rows, (uint64_t)d.K, (uint64_t)d.lda, kBM, kBK)) {
@@ -259,7 +258,9 @@ cudaError_t gemm_bf16_tn(const GemmDesc& d, cudaStream_t stream) {
     return cudaErrorInvalidValue;
   // Many result rows: the CTA-pair kernel, whose result is row-major (with trans_out the rows are B's; a dual or packed A
   // can only be its B operand, so those need trans_out).
-  const bool width_ok = d.bn == 0 || d.bn == 64 || d.bn == 128 || d.bn == 256 || (d.bn > 64 && d.bn < 256 && d.bn % 32 == 0 && !d.a_tiled && d.dual_off == 0);
+  if (d.a_tiled && d.dual_off % gemm::kBM != 0) return cudaErrorInvalidValue;  // gate and up start on whole packed tiles
+  const bool width_ok = d.bn == 0 || d.bn == 64 || d.bn == 128 || (d.bn == 256 && d.dual_off == 0) ||
+                        (d.bn > 64 && d.bn < 256 && d.bn % 32 == 0 && !d.a_tiled && d.dual_off == 0);
   if (width_ok && d.splitk <= 1 && (d.trans_out ? d.N : d.M) > 128 && (d.trans_out || (!d.a_tiled && d.dual_off == 0)))
     return gemm::dispatch_2sm(d, stream);
   int bn = d.bn;
