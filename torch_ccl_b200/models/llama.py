@@ -232,9 +232,7 @@ class TPLlamaDecoder:
         out.copy_(rows * ok[:, None].to(rows.dtype))
 
     def _decode_body(self, B):
-        if self._fused_rows(B):
-            return self._decode_body_fused(B)
-        return self._decode_body_unfused(B)
+        return self._decode_body_fused(B) if self.fused else self._decode_body_unfused(B)
 
     def _fused_rows(self, B):
         return self.fused and self.comm.fits_gemm_ar_norm(self.h, B, self.cfg.hidden, self.inter)
@@ -267,8 +265,9 @@ class TPLlamaDecoder:
         cfg = self.cfg
         tokens, h, xn = self.tokens[:B], self.h[:B], self.xn[:B]
         self.comm.embed_norm(tokens, self.embed, self.rank * self.vshard, h, self.layers[0]["attn_norm"], xn, cfg.eps)
+        layer = self._layer_fused if self._fused_rows(B) else self._layer_unfused
         for li, L in enumerate(self.layers):
-            self._layer_fused(li, B, L["k"], L["v"], self.positions[:B])
+            layer(li, B, L["k"], L["v"], self.positions[:B])
         self._gemm_t(self.lm_head, xn, self.logits[:B], self.vshard)
         # feeds the sampled ids back into self.tokens and advances the positions: steady state is a pure replay
         self.comm.sample(self.logits[:B], self.next_tokens[:B], tokens, self.positions[:B])
