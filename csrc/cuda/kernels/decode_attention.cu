@@ -2,9 +2,16 @@
 // the KV-cache append: one launch per layer reads q/k/v of the new token from the packed QKV
 // projection output, rotates q and k, writes k/v into the cache at the sequence's current
 // position, and attends over positions [0, pos]. Memory-bound on the KV cache, so the work is
-// split over the sequence (flash-decoding): each CTA handles one (sequence, head, KV range) and
-// writes an un-normalised partial (running max, sum, output) to a scratch buffer; the last CTA
-// to finish a (sequence, head) combines the partials. head_dim is fixed at 128.
+// split over the sequence (flash-decoding): each CTA handles one (sequence, G heads, KV range) and
+// writes an un-normalised partial (running max, sum, output) per head to a scratch buffer; the last
+// CTA to finish a range's heads combines the partials. head_dim is fixed at 128.
+//
+// G heads that share a KV head (grouped-query attention) go through one CTA together: K and V then
+// cross from L2 once for all of them and are widened to fp32 once, while each head keeps the
+// arithmetic and its order, so that a result does not depend on G (33 sequences of up to 3000
+// positions, 32 heads on 8: 150 -> 121 us, then bound by instructions). The sums stay on the CUDA
+// cores: tensor cores, with three bf16 parts per fp32 value, took 53-80 us there, but another order
+// of the sums moves the results of 32 layers by 2 % through the bf16 roundings in between.
 //
 // The K and V rows of one (sequence, head) are contiguous in the cache, so one elected thread
 // streams them with untiled bulk copies (cp.async.bulk, completion on an mbarrier) into a 3-stage
@@ -78,10 +85,11 @@ __device__ __forceinline__ void rope16(float (&own)[16], const float (&partner)[
   }
 }
 
+template <int G>
 __global__ void __launch_bounds__(kThreads) decode_attention_kernel(const DecodeAttnParams p) {
   ptx::griddep_launch_dependents();
   const int split = blockIdx.x;
-  const int h = blockIdx.y;
+  const int h = blockIdx.y * G;  // the first of this CTA's heads
   const int b = blockIdx.z;
   const int nsplit = gridDim.x;
   const int tid = threadIdx.x;
@@ -113,7 +121,8 @@ __global__ void __launch_bounds__(kThreads) decode_attention_kernel(const Decode
     // record it, write nothing to the cache and emit a zero row (uniform for the whole CTA, and
     // every split of this (sequence, head) takes the same exit, so the arrival counter stays 0)
     if (tid == 0 && p.status) atomicExch(p.status, 201);
-    if (split == 0) p.out[(size_t)b * p.out_stride + (size_t)h * kHD + tid] = __float2bfloat16(0.f);
+    if (split == 0)
+      for (int e = 0; e < G; ++e) p.out[(size_t)b * p.out_stride + (size_t)(h + e) * kHD + tid] = __float2bfloat16(0.f);
     return;
   }
   const int total = pos + 1;
@@ -127,14 +136,15 @@ __global__ void __launch_bounds__(kThreads) decode_attention_kernel(const Decode
   const int pj = j ^ 4;
 
   // q: rotate and pre-scale
-  float q[16];
-  {
-    float partner[16];
-    load16(qkv + (size_t)h * kHD + j * 16, q);
-    load16(qkv + (size_t)h * kHD + pj * 16, partner);
-    rope16(q, partner, cosr, sinr, j);
+  float q[G][16];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) q[i] *= p.scale;
+  for (int e = 0; e < G; ++e) {
+    float partner[16];
+    load16(qkv + (size_t)(h + e) * kHD + j * 16, q[e]);
+    load16(qkv + (size_t)(h + e) * kHD + pj * 16, partner);
+    rope16(q[e], partner, cosr, sinr, j);
+#pragma unroll
+    for (int i = 0; i < 16; ++i) q[e][i] *= p.scale;
   }
 
   __nv_bfloat16* kc = p.k_cache + (((size_t)b * p.n_kv_heads + kvh) * p.max_seq) * kHD;
@@ -142,7 +152,7 @@ __global__ void __launch_bounds__(kThreads) decode_attention_kernel(const Decode
 
   // The CTA whose range contains `pos` handles the new token from the projection output: it
   // rotates k, keeps k/v (rounded like the cache) in shared memory for its own use and, for the
-  // first head of a KV group, appends them to the cache. No other CTA reads that position.
+  // first heads of a KV group, appends them to the cache. No other CTA reads that position.
   const bool owns_new = (pos >= t0 && pos < t1);
   __shared__ float s_new_k[kHD], s_new_v[kHD];
   if (owns_new && g == 0) {
@@ -166,9 +176,14 @@ __global__ void __launch_bounds__(kThreads) decode_attention_kernel(const Decode
   __syncthreads();
 
   const unsigned gmask = 0xffu << (8 * ((tid & 31) >> 3));
-  float m = -INFINITY, l = 0.f, o[16];
+  float m[G], l[G], o[G][16];
 #pragma unroll
-  for (int i = 0; i < 16; ++i) o[i] = 0.f;
+  for (int e = 0; e < G; ++e) {
+    m[e] = -INFINITY;
+    l[e] = 0.f;
+#pragma unroll
+    for (int i = 0; i < 16; ++i) o[e][i] = 0.f;
+  }
 
   // ---- stream [t0, t1) through the shared-memory ring ---------------------------------------
   extern __shared__ __align__(128) unsigned char dyn_smem[];
@@ -219,19 +234,27 @@ __global__ void __launch_bounds__(kThreads) decode_attention_kernel(const Decode
       }
       // all 8 lanes of a group share `lt`, so the branch is uniform within the shuffle mask
       if (lt < n) {
-        float s = 0.f;
+        float s[G];
 #pragma unroll
-        for (int i = 0; i < 16; ++i) s += q[i] * k[i];
-        s += __shfl_xor_sync(gmask, s, 1);
-        s += __shfl_xor_sync(gmask, s, 2);
-        s += __shfl_xor_sync(gmask, s, 4);
-        const float mn = fmaxf(m, s);
-        const float corr = __expf(m - mn);
-        const float pr = __expf(s - mn);
-        l = l * corr + pr;
+        for (int e = 0; e < G; ++e) {
+          s[e] = 0.f;
 #pragma unroll
-        for (int i = 0; i < 16; ++i) o[i] = o[i] * corr + pr * v[i];
-        m = mn;
+          for (int i = 0; i < 16; ++i) s[e] += q[e][i] * k[i];
+        }
+#pragma unroll
+        for (int x = 1; x <= 4; x *= 2)
+#pragma unroll
+          for (int e = 0; e < G; ++e) s[e] += __shfl_xor_sync(gmask, s[e], x);
+#pragma unroll
+        for (int e = 0; e < G; ++e) {
+          const float mn = fmaxf(m[e], s[e]);
+          const float corr = __expf(m[e] - mn);
+          const float pr = __expf(s[e] - mn);
+          l[e] = l[e] * corr + pr;
+#pragma unroll
+          for (int i = 0; i < 16; ++i) o[e][i] = o[e][i] * corr + pr * v[i];
+          m[e] = mn;
+        }
       }
     }
     __syncthreads();  // everyone is done with this stage: refill it
@@ -242,36 +265,44 @@ __global__ void __launch_bounds__(kThreads) decode_attention_kernel(const Decode
   // combine the kGroups position groups of this CTA
   // (the ring is free now — every chunk was consumed before the last barrier — and is reused
   // for the partial outputs)
-  __shared__ float s_m[kGroups], s_l[kGroups];
-  float (*s_o)[kHD] = reinterpret_cast<float (*)[kHD]>(ring);
-  if (j == 0) {
-    s_m[g] = m;
-    s_l[g] = l;
-  }
+  static_assert((size_t)G * kGroups * kHD * 4 <= (size_t)kStages * kStageBytes, "the partial outputs fit the ring");
+  __shared__ float s_m[G][kGroups], s_l[G][kGroups];
+  float (*s_o)[kGroups][kHD] = reinterpret_cast<float (*)[kGroups][kHD]>(ring);
 #pragma unroll
-  for (int i = 0; i < 16; ++i) s_o[g][j * 16 + i] = o[i];
+  for (int e = 0; e < G; ++e) {
+    if (j == 0) {
+      s_m[e][g] = m[e];
+      s_l[e][g] = l[e];
+    }
+#pragma unroll
+    for (int i = 0; i < 16; ++i) s_o[e][g][j * 16 + i] = o[e][i];
+  }
   __syncthreads();
-  float M = -INFINITY;
-  for (int i = 0; i < kGroups; ++i) M = fmaxf(M, s_m[i]);
-  float L = 0.f, acc = 0.f;  // thread `tid` owns output dim tid
-  for (int i = 0; i < kGroups; ++i) {
-    const float w = (s_m[i] == -INFINITY) ? 0.f : __expf(s_m[i] - M);
-    L += s_l[i] * w;
-    acc += s_o[i][tid] * w;
-  }
-
   __nv_bfloat16* out = p.out + (size_t)b * p.out_stride + (size_t)h * kHD;
-  if (nsplit == 1) {
-    out[tid] = __float2bfloat16(acc / L);
-    return;
-  }
   // partial of this split: [b][h][split] -> {M, L, o[128]}
+  const size_t head_stride = (size_t)nsplit * (kHD + 2);
   float* part = p.scratch + (((size_t)b * p.n_heads + h) * nsplit + split) * (kHD + 2);
-  part[2 + tid] = acc;
-  if (tid == 0) {
-    part[0] = M;
-    part[1] = L;
+#pragma unroll
+  for (int e = 0; e < G; ++e) {
+    float M = -INFINITY;
+    for (int i = 0; i < kGroups; ++i) M = fmaxf(M, s_m[e][i]);
+    float L = 0.f, acc = 0.f;  // thread `tid` owns output dim tid
+    for (int i = 0; i < kGroups; ++i) {
+      const float w = (s_m[e][i] == -INFINITY) ? 0.f : __expf(s_m[e][i] - M);
+      L += s_l[e][i] * w;
+      acc += s_o[e][i][tid] * w;
+    }
+    if (nsplit == 1) {
+      out[e * kHD + tid] = __float2bfloat16(acc / L);
+      continue;
+    }
+    part[e * head_stride + 2 + tid] = acc;
+    if (tid == 0) {
+      part[e * head_stride] = M;
+      part[e * head_stride + 1] = L;
+    }
   }
+  if (nsplit == 1) return;
   __threadfence();
   __shared__ int s_last;
   __syncthreads();
@@ -284,18 +315,41 @@ __global__ void __launch_bounds__(kThreads) decode_attention_kernel(const Decode
   __syncthreads();
   if (!s_last) return;
   __threadfence();
-  const float* base = p.scratch + ((size_t)b * p.n_heads + h) * nsplit * (kHD + 2);
-  float GM = -INFINITY;
-  for (int i = 0; i < nsplit; ++i) GM = fmaxf(GM, __ldcg(base + (size_t)i * (kHD + 2)));
-  float GL = 0.f, gacc = 0.f;
-  for (int i = 0; i < nsplit; ++i) {
-    const float* pi = base + (size_t)i * (kHD + 2);
-    const float mi = __ldcg(pi);
-    const float w = (mi == -INFINITY) ? 0.f : __expf(mi - GM);
-    GL += __ldcg(pi + 1) * w;
-    gacc += __ldcg(pi + 2 + tid) * w;
+#pragma unroll
+  for (int e = 0; e < G; ++e) {
+    const float* base = p.scratch + ((size_t)b * p.n_heads + h + e) * head_stride;
+    float GM = -INFINITY;
+    for (int i = 0; i < nsplit; ++i) GM = fmaxf(GM, __ldcg(base + (size_t)i * (kHD + 2)));
+    float GL = 0.f, gacc = 0.f;
+    for (int i = 0; i < nsplit; ++i) {
+      const float* pi = base + (size_t)i * (kHD + 2);
+      const float mi = __ldcg(pi);
+      const float w = (mi == -INFINITY) ? 0.f : __expf(mi - GM);
+      GL += __ldcg(pi + 1) * w;
+      gacc += __ldcg(pi + 2 + tid) * w;
+    }
+    out[e * kHD + tid] = __float2bfloat16(gacc / GL);
   }
-  out[tid] = __float2bfloat16(gacc / GL);
+}
+
+template <int G>
+cudaError_t launch(const DecodeAttnParams& p, int batch, int nsplit, cudaStream_t stream) {
+  auto kern = decode_attention_kernel<G>;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nsplit, p.n_heads / G, batch);
+  cfg.blockDim = dim3(kThreads, 1, 1);
+  static DeviceOnce configured;  // the shared-memory opt-in is a per-device attribute
+  if (configured.pending()) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynSmem);
+    if (e != cudaSuccess) return e;
+    configured.done();
+  }
+  cfg.dynamicSmemBytes = kDynSmem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  cfg.attrs = attr;
+  cfg.numAttrs = pdl_launch_attr(&attr[0]);
+  return cudaLaunchKernelEx(&cfg, kern, p);
 }
 
 }  // namespace
@@ -329,30 +383,24 @@ bool decode_attention_layout_ok(const DecodeAttnParams& p) {
   return true;
 }
 
+// Heads of one KV head that share a CTA: two where two CTAs per SM remain, measured (us, one / two / four heads a CTA): 33
+// sequences of up to 3000 positions, 32 heads on 8, 150 / 121 / 125; all of 3000, 201 / 127 / 127; 100 of up to 300 on 4, 54 / 39 /
+// 43; but one sequence of 4001 positions, whose 512 CTAs would become 256, 17.4 / 22.5 / 27.4. Four heads take 219 registers.
+static int heads_per_cta(int n_heads, int n_kv_heads, int batch, int nsplit) {
+  if (n_kv_heads <= 0 || n_heads % n_kv_heads != 0 || (n_heads / n_kv_heads) % 2 != 0) return 1;
+  return (long long)batch * (n_heads / 2) * nsplit >= 2 * 148 ? 2 : 1;
+}
+
 cudaError_t decode_attention(const DecodeAttnParams& p, int batch, int nsplit, cudaStream_t stream) {
   if (p.head_dim != kHD) return cudaErrorInvalidValue;
   if (nsplit > 1 && (!p.scratch || !p.counters)) return cudaErrorInvalidValue;
   if (!decode_attention_layout_ok(p)) return cudaErrorInvalidValue;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nsplit, p.n_heads, batch);
-  cfg.blockDim = dim3(kThreads, 1, 1);
-  static DeviceOnce configured;  // the shared-memory opt-in is a per-device attribute
-  if (configured.pending()) {
-    cudaError_t e = cudaFuncSetAttribute(decode_attention_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDynSmem);
-    if (e != cudaSuccess) return e;
-    configured.done();
-  }
-  cfg.dynamicSmemBytes = kDynSmem;
-  cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  cfg.attrs = attr;
-  cfg.numAttrs = pdl_launch_attr(&attr[0]);
   // Early L2 prefetch only when the K/V of the whole launch is well below the 126 MB L2 (a tensor-parallel
   // shard): for a full-size cache (268 MB at batch 16 x 32 heads) the hint would only evict itself and was
   // measured to cost 20 % of the step.
   DecodeAttnParams q = p;
   q.prefetch_l2 = pdl_enabled() && (size_t)batch * p.n_kv_heads * p.max_seq * kRowBytes * 2 <= (48u << 20);
-  return cudaLaunchKernelEx(&cfg, decode_attention_kernel, q);
+  return heads_per_cta(p.n_heads, p.n_kv_heads, batch, nsplit) == 2 ? launch<2>(q, batch, nsplit, stream) : launch<1>(q, batch, nsplit, stream);
 }
 
 }  // namespace ccl
