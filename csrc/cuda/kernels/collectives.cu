@@ -1031,10 +1031,14 @@ __global__ void __launch_bounds__(512) allreduce_residual_rmsnorm_kernel(const _
 // a row's bytes (x, residual in and out, out; the weight stays in cache). One CTA per row; every thread requests its
 // vectors of x and of the residual before it uses one. The kernel above walks 64 rows per CTA, one block barrier after
 // the other, with one or two CTAs per SM: 16384 x 4096 bf16 took 351 us there.
+// The sum of squares has the order of the kernel above, whose CTA is min(512, hidden / 8 rounded up to a warp) threads
+// wide: each thread here stands for V of its threads, blockDim apart, keeps their sums apart and reduces them warp by
+// warp. So a row's result does not depend on how many rows there are, or on which of the two kernels made it.
 // ---------------------------------------------------------------------------------------------
-template <typename T, int MV>
+template <typename T, int MV, int V>
 __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(const FusedNormArgs a) {
-  __shared__ float s_red[33];
+  static_assert(MV % V == 0, "whole rounds of the threads stood for");
+  __shared__ float s_red[17];
   ptx::griddep_launch_dependents();
   const int hv = a.hidden / 8;
   const int row = blockIdx.x;
@@ -1057,7 +1061,9 @@ __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(const FusedNormAr
     *reinterpret_cast<uint4*>(&xv[k]) = (x && i < hv) ? *reinterpret_cast<const uint4*>(x + (size_t)i * 16) : make_uint4(0, 0, 0, 0);
     *reinterpret_cast<uint4*>(&hn[k]) = (!a.zero_residual && i < hv) ? *reinterpret_cast<const uint4*>(res + (size_t)i * 16) : make_uint4(0, 0, 0, 0);
   }
-  float ss = 0.f;
+  float ss[V];
+#pragma unroll
+  for (int j = 0; j < V; ++j) ss[j] = 0.f;
 #pragma unroll
   for (int k = 0; k < MV; ++k) {
     const int i = threadIdx.x + k * blockDim.x;
@@ -1065,11 +1071,26 @@ __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(const FusedNormAr
     for (int t = 0; t < 8; ++t) {
       hn[k].v[t] = a.zero_residual ? xv[k].v[t] : ll_round_to<T>(to_acc(xv[k].v[t]) + to_acc(hn[k].v[t]));
       const float h = to_acc(hn[k].v[t]);
-      ss += h * h;
+      ss[k % V] += h * h;
     }
     if (i < hv) *reinterpret_cast<uint4*>(res + (size_t)i * 16) = *reinterpret_cast<const uint4*>(&hn[k]);
   }
-  const float rstd = rsqrtf(block_sum(ss, s_red) / (float)a.hidden + a.eps);
+  const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
+#pragma unroll
+  for (int j = 0; j < V; ++j) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], o);
+    if ((threadIdx.x & 31) == 0) s_red[j * nwarp + warp] = ss[j];
+  }
+  __syncthreads();
+  if (warp == 0) {
+    float t = (int)threadIdx.x < V * nwarp ? s_red[threadIdx.x] : 0.f;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+    if (threadIdx.x == 0) s_red[16] = t;
+  }
+  __syncthreads();
+  const float rstd = rsqrtf(s_red[16] / (float)a.hidden + a.eps);
   ll_row_write_norm<T, MV>(hn, wv, rstd, 0, hv, static_cast<char*>(a.out) + (size_t)row * row_bytes);
 }
 
@@ -1079,8 +1100,9 @@ cudaError_t launch_residual_rmsnorm(const FusedNormArgs& a, cudaStream_t stream)
   // flight on an SM (the crossover is where one CTA per SM of the wide form no longer covers the rows).
   const int hv = a.hidden / 8;
   const bool many = a.rows > 4 * 148 || hv > 512;
-  const int mv = many ? 4 : 1;
-  const int threads = std::max(32, ((hv + mv - 1) / mv + 31) / 32 * 32);
+  // More than 512 vectors go round the 512 threads stood for twice (V = 2, 256 threads) or up to four times (V = 1).
+  const int v = !many || hv > 1024 ? 1 : (hv > 512 ? 2 : 4);
+  const int threads = hv > 512 ? 512 / v : std::max(32, ((hv + v - 1) / v + 31) / 32 * 32);
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(a.rows, 1, 1);
   lc.blockDim = dim3(threads, 1, 1);
@@ -1088,7 +1110,9 @@ cudaError_t launch_residual_rmsnorm(const FusedNormArgs& a, cudaStream_t stream)
   cudaLaunchAttribute attr[1];
   lc.attrs = attr;
   lc.numAttrs = pdl_launch_attr(&attr[0]);
-  return many ? cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 4>, a) : cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 1>, a);
+  if (!many) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 1, 1>, a);
+  if (v == 4) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 4, 4>, a);
+  return v == 2 ? cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 4, 2>, a) : cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 4, 1>, a);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -31,6 +31,23 @@ def test_residual_rmsnorm(comm, rows, hidden, dtype):
     torch.testing.assert_close(out.float(), n.float() * w.float(), rtol=3 * half, atol=1e-6)
 
 
+@pytest.mark.parametrize("rows,hidden", [(2, 4096), (593, 952), (700, 4096), (5, 4104), (600, 5120), (600, 8192), (600, 8200), (600, 16384)])
+def test_residual_rmsnorm_sums_in_the_order_of_the_staged_kernel(comm, rows, hidden):
+    """Bit for bit what the kernel for several ranks gives for one (the emulation takes that one)."""
+    import torch_ccl_b200._C as C
+
+    g = torch.Generator(device="cuda").manual_seed(rows * hidden)
+    x, res, w = (torch.randn(*s, generator=g, device="cuda").bfloat16() for s in ((rows, hidden), (rows, hidden), (hidden,)))
+    # one element carries most of a row's sum, so that the order of the small ones shows in its last bits
+    x[:, 0] = 64.0
+    got = []
+    for c in (comm, C.CudaComm.emulated(1, 1 << 20, 1000, 8)):
+        r, out = res.clone(), torch.empty_like(x)
+        c.allreduce_residual_rmsnorm([x], [r], [w], [out], 1e-5)
+        got.append((r, out))
+    assert torch.equal(got[0][0], got[1][0]) and torch.equal(got[0][1], got[1][1])
+
+
 def test_residual_rmsnorm_embedding(comm):
     """Token ids outside this rank's part of the table contribute zeros; the residual is not read."""
     table = torch.randn(50, 256, device="cuda").bfloat16()
