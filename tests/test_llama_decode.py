@@ -100,3 +100,19 @@ def test_prefill_matches_token_by_token():
     for L1, L2 in zip(m1.layers, m2.layers):
         torch.testing.assert_close(L1["k"][:, :, :S].float(), L2["k"][:, :, :S].float(), rtol=5e-2, atol=5e-2)
         torch.testing.assert_close(L1["v"][:, :, :S].float(), L2["v"][:, :, :S].float(), rtol=5e-2, atol=5e-2)
+
+
+@pytest.mark.parametrize("n,S", [(1, 40), (3, 150)])
+def test_prefill_fills_every_position_alike(n, S):
+    """What the caches hold for a position does not depend on whether it is the prompt's last one, nor on the sequences
+    that are prefilled with it."""
+    ids = torch.randint(0, 1024, (n, S + 1), generator=torch.Generator().manual_seed(5))
+    caches, tokens = [], []
+    for prompt, chunk in ((ids, None), (ids[:, :S], None), (ids[:, :S], 1)):
+        m = _model(batch=n, max_seq=256, layers=1)
+        m.prefill(prompt, chunk_seqs=chunk)
+        caches.append([m.layers[0][c][:, :, :S].clone() for c in "kv"])
+        tokens.append(m.tokens[:n].clone())
+    for other in caches[1:]:
+        assert all(torch.equal(a, b) for a, b in zip(caches[0], other))
+    assert torch.equal(tokens[1], tokens[2])

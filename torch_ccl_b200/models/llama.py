@@ -341,8 +341,9 @@ class TPLlamaDecoder:
         rows per GEMM): the tcgen05 GEMM on CTA pairs with the weights as its B operand, one pass for rotary
         embedding and KV append, torch's scaled_dot_product_attention for the causal attention over the prompt
         itself (reading K and V where they stay), the all_reduce fused with residual add + norm (in slices that fit
-        the communicator's staging arena). Of the last layer only K and V are wanted for every position; the
-        rest of it runs for the last position of each sequence, as the decode step does.
+        the communicator's staging arena). After the attention of the last layer only the last position of each
+        sequence is wanted: the rest of that layer runs for those rows alone, with the sums over K in the order that
+        they have for all rows (no split), so that a prompt's results do not depend on the shortcut.
         `chunk_seqs` bounds the sequences per pass (default: as many as keep a pass under ~32k rows)."""
         cfg = self.cfg
         B, S = prompt.shape
@@ -353,22 +354,20 @@ class TPLlamaDecoder:
         cap_rows = 1024 if self.world > 1 else 1 << 30  # rows per fused-norm launch (staging capacity)
         per = chunk_seqs or max(1, 32768 // S)
         last_li = cfg.n_layers - 1
-        # the packed rows of K and V within wqkv: whole 128-row tiles after those of q
-        kv_off = nq * ((H + 63) // 64)
         for b0 in range(0, B, per):
             n = min(per, B - b0)
             R = n * S
             toks = prompt[b0:b0 + n].reshape(-1).to(dev)
             h = torch.empty(R, H, **bf)
             xn = torch.empty(R, H, **bf)
-            if last_li > 0 or self.comm.nccl is not None:
-                x = torch.empty(R, H, **bf)
-                qkv = torch.empty(R, nq + 2 * nkv, **bf)
-                act = torch.empty(R, self.inter, **bf)
+            x = torch.empty(R, H, **bf)
+            qkv = torch.empty(R, nq + 2 * nkv, **bf)
+            act = torch.empty(R, self.inter, **bf)
 
             def norm_step(w):
-                for r0 in range(0, R, cap_rows):
-                    r1 = min(R, r0 + cap_rows)
+                rows = x.shape[0]
+                for r0 in range(0, rows, cap_rows):
+                    r1 = min(rows, r0 + cap_rows)
                     self.comm.ar_res_norm(x[r0:r1], h[r0:r1], w, xn[r0:r1], cfg.eps)
 
             if self.comm.nccl is not None:  # comparison arm: the lookup is reduced by NCCL
@@ -380,29 +379,26 @@ class TPLlamaDecoder:
                     r1 = min(R, r0 + cap_rows)
                     self.comm.embed_norm(toks[r0:r1], self.embed, self.rank * self.vshard, h[r0:r1], self.layers[0]["attn_norm"],
                                          xn[r0:r1], cfg.eps)
-            for li, L in enumerate(self.layers[:last_li]):
+            splitk = 0
+            for li, L in enumerate(self.layers):
                 k, v = L["k"][b0:b0 + n], L["v"][b0:b0 + n]
                 self._gemm_t(L["wqkv"], xn, qkv, self.qkv_rows)
                 _C.rope_append(qkv, k, v, self.cos, self.sin, self.nh, S)
                 o = torch.nn.functional.scaled_dot_product_attention(
                     qkv.view(n, S, -1)[..., :nq].view(n, S, self.nh, hd).transpose(1, 2), k[:, :, :S], v[:, :, :S], is_causal=True,
-                    enable_gqa=self.nh != self.nkv)
-                self._gemm_t(L["wo"], o.transpose(1, 2).reshape(R, nq), x, H)
+                    enable_gqa=self.nh != self.nkv).transpose(1, 2)
+                # (a chunk of at most 128 rows is one tile of rows, whatever is left out of it: it stays as it is)
+                if li == last_li and R > 128:
+                    o, h = o[:, S - 1], h.view(n, S, H)[:, S - 1].contiguous()
+                    x, xn, act, splitk = x[:n], xn[:n], act[:n], 1
+                self._gemm_t(L["wo"], o.reshape(-1, nq), x, H, splitk=splitk)
                 norm_step(L["mlp_norm"])
-                self._gemm_t(L["wgu"], xn, act, self.inter, dual=self.inter_pad)
-                self._gemm_t(L["wd"], act, x, H)
+                self._gemm_t(L["wgu"], xn, act, self.inter, dual=self.inter_pad, splitk=splitk)
+                self._gemm_t(L["wd"], act, x, H, splitk=splitk)
                 norm_step(self._next_norm(li))
-            L = self.layers[last_li]
-            k, v = L["k"][b0:b0 + n], L["v"][b0:b0 + n]
-            kv = torch.empty(R, 2 * nkv, **bf)
-            self._gemm_t(L["wqkv"][kv_off:], xn, kv, 2 * nkv)
-            _C.rope_append(kv, k, v, self.cos, self.sin, 0, S)
-            self.h[:n].copy_(h.view(n, S, H)[:, S - 1])
-            self.xn[:n].copy_(xn.view(n, S, H)[:, S - 1])
-            (self._layer_fused if self._fused_rows(n) else self._layer_unfused)(
-                last_li, n, k, v, torch.full((n,), S - 1, device=dev, dtype=torch.int32))
+            last = xn if R > 128 else xn.view(n, S, H)[:, S - 1].contiguous()
             logits = torch.empty(n, self.vshard, device=dev, dtype=torch.float32)
-            self._gemm_t(self.lm_head, self.xn[:n], logits, self.vshard)
+            self._gemm_t(self.lm_head, last, logits, self.vshard)
             val, idx = logits.max(dim=-1)
             if self.world > 1:
                 mine = torch.stack([val, (idx + self.rank * self.vshard).float()], dim=-1).contiguous()
