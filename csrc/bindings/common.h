@@ -22,7 +22,7 @@ ccl::FusedNormArgs make_norm_args(const at::Tensor& x, at::Tensor& residual, con
 ccl::GemmArNormArgs make_gemm_ar_norm_args(const at::Tensor& w_packed, const at::Tensor& x, at::Tensor& residual,
                                            const at::Tensor& weight, at::Tensor& out, double eps, int64_t splitk);
 ccl::SampleArgs make_sample_args(const at::Tensor& logits, at::Tensor& next_tokens, const c10::optional<at::Tensor>& tokens,
-                                 const c10::optional<at::Tensor>& positions);
+                                 const c10::optional<at::Tensor>& positions, bool nan_first);
 void bind_cuda_comm(py::module& m);
 void bind_process_group(py::module& m);
 void bind_model_ops(py::module& m);

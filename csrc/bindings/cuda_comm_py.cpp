@@ -141,7 +141,7 @@ ccl::GemmArNormArgs make_gemm_ar_norm_args(const at::Tensor& w_packed, const at:
 }
 
 ccl::SampleArgs make_sample_args(const at::Tensor& logits, at::Tensor& next_tokens, const c10::optional<at::Tensor>& tokens,
-                                 const c10::optional<at::Tensor>& positions) {
+                                 const c10::optional<at::Tensor>& positions, bool nan_first) {
   TORCH_CHECK(logits.is_cuda() && logits.scalar_type() == at::kFloat && logits.dim() == 2 && logits.stride(1) == 1, "sample: logits must be [rows, vocab shard] fp32");
   TORCH_CHECK(next_tokens.is_cuda() && next_tokens.device() == logits.device() && next_tokens.scalar_type() == at::kLong &&
                   next_tokens.is_contiguous() && next_tokens.numel() >= logits.size(0), "sample: next_tokens must be int64 [rows]");
@@ -150,6 +150,7 @@ ccl::SampleArgs make_sample_args(const at::Tensor& logits, at::Tensor& next_toke
   a.ld = logits.stride(0);
   a.vshard = (int)logits.size(1);
   a.rows = (int)logits.size(0);
+  a.nan_first = nan_first;
   a.next_tokens = reinterpret_cast<long long*>(next_tokens.data_ptr<int64_t>());
   if (tokens.has_value()) {
     TORCH_CHECK(tokens->is_cuda() && tokens->device() == logits.device() && tokens->scalar_type() == at::kLong && tokens->is_contiguous() &&
@@ -345,14 +346,14 @@ struct PyComm {
   }
 
   void sample_allgather(std::vector<at::Tensor> logits, std::vector<at::Tensor> next_tokens,
-                        c10::optional<std::vector<at::Tensor>> tokens, c10::optional<std::vector<at::Tensor>> positions) {
+                        c10::optional<std::vector<at::Tensor>> tokens, c10::optional<std::vector<at::Tensor>> positions, bool nan_first) {
     check_n(logits.size());
     std::vector<ccl::SampleArgs> args(logits.size());
     for (size_t i = 0; i < logits.size(); ++i) {
       c10::optional<at::Tensor> t, p;
       if (tokens.has_value()) t = (*tokens)[i];
       if (positions.has_value()) p = (*positions)[i];
-      args[i] = make_sample_args(logits[i], next_tokens[i], t, p);
+      args[i] = make_sample_args(logits[i], next_tokens[i], t, p, nan_first);
     }
     cu(comm->sample_allgather(args, stream()), "sample_allgather");
   }
@@ -608,7 +609,7 @@ void bind_cuda_comm(py::module& m) {
            py::arg("eps"), py::arg("splitk") = 0)
       .def("fits_gemm_ar_norm", [](PyComm& c, int rows, int hidden, int k) { return c.comm->fits_gemm_ar_norm(rows, hidden, k); })
       .def("sample_allgather", &PyComm::sample_allgather, py::arg("logits"), py::arg("next_tokens"), py::arg("tokens") = py::none(),
-           py::arg("positions") = py::none())
+           py::arg("positions") = py::none(), py::arg("nan_first") = false)
       .def("multi", &PyComm::multi, py::arg("mode"), py::arg("ins"), py::arg("outs"), py::arg("op") = 0, py::arg("scale") = 1.0,
            py::arg("has_scale") = 0)
       .def("symm_empty", &PyComm::symm_empty)

@@ -42,10 +42,10 @@ void gemm_ar_norm(ProcessGroupCCL& pg, const at::Tensor& w_packed, const at::Ten
 }
 
 void sample_allgather(ProcessGroupCCL& pg, const at::Tensor& logits, at::Tensor& next_tokens,
-                      const c10::optional<at::Tensor>& tokens, const c10::optional<at::Tensor>& positions) {
+                      const c10::optional<at::Tensor>& tokens, const c10::optional<at::Tensor>& positions, bool nan_first) {
   auto& c = cuda_comm_of(pg, logits);
   c10::cuda::CUDAGuard g(logits.device());
-  ccl::SampleArgs a = ccl_py::make_sample_args(logits, next_tokens, tokens, positions);
+  ccl::SampleArgs a = ccl_py::make_sample_args(logits, next_tokens, tokens, positions, nan_first);
   C10_CUDA_CHECK(c.sample_allgather({a}, c10::cuda::getCurrentCUDAStream()));
 }
 

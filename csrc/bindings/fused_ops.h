@@ -18,7 +18,7 @@ void allreduce_residual_rmsnorm(ProcessGroupCCL& pg, const at::Tensor& x, at::Te
 void gemm_ar_norm(ProcessGroupCCL& pg, const at::Tensor& w_packed, const at::Tensor& x, at::Tensor& residual,
                   const at::Tensor& weight, at::Tensor& out, double eps, int64_t splitk);
 void sample_allgather(ProcessGroupCCL& pg, const at::Tensor& logits, at::Tensor& next_tokens,
-                      const c10::optional<at::Tensor>& tokens, const c10::optional<at::Tensor>& positions);
+                      const c10::optional<at::Tensor>& tokens, const c10::optional<at::Tensor>& positions, bool nan_first);
 void all_reduce_scaled(ProcessGroupCCL& pg, at::Tensor& t, double scale);
 void reduce_scatter_cast(ProcessGroupCCL& pg, const at::Tensor& inp, at::Tensor& out, double scale);
 // dst[offsets[i] ...] += scale * src[i] for tensors of one dtype (bf16 / f16 / f32; dst: the same or fp32), in one launch.

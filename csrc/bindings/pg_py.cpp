@@ -98,7 +98,7 @@ void bind_process_group(py::module& m) {
       })
       // arg-max over the local logits shard + all-gather of the winners; writes the global winner ids
       .def("fused_sample_allgather", &ccl_ops::sample_allgather, py::arg("logits"), py::arg("next_tokens"), py::arg("tokens") = py::none(),
-           py::arg("positions") = py::none())
+           py::arg("positions") = py::none(), py::arg("nan_first") = false)
       .def("fused_allreduce", &ccl_ops::all_reduce_scaled, py::arg("tensor"), py::arg("scale") = 1.0)
       // out (fp32 or input dtype) = scale * sum over ranks of this rank's piece of `inp`
       .def("fused_reduce_scatter_cast", &ccl_ops::reduce_scatter_cast, py::arg("input"), py::arg("output"), py::arg("scale") = 1.0)

@@ -175,8 +175,9 @@ struct LaunchSample {
   SampleArgs args_table[EMU ? kMaxRanks : 1];
 };
 
-__device__ __forceinline__ void better(float& v, int& i, float ov, int oi) {
-  if (ov > v || (ov == v && oi < i)) {
+// Ties go to the lower index. With nan_first a NaN is above everything, and the first one wins (as torch.max has it).
+__device__ __forceinline__ void better(float& v, int& i, float ov, int oi, bool nan_first) {
+  if (ov > v || (ov == v && oi < i) || (nan_first && ov != ov && (v == v || oi < i))) {
     v = ov;
     i = oi;
   }
@@ -193,6 +194,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_allgather_kernel(const 
   const int W = ctx.world, me = ctx.rank;
   const int row = blockIdx.x;
   const float* lg = a.logits + (size_t)row * a.ld;
+  const bool nf = a.nan_first != 0;
   float bv = -INFINITY;
   int bi = 0x7fffffff;
   // One CTA per row, so what counts is how many loads it has in flight: eight 16-byte vectors a thread, the elements before the
@@ -201,7 +203,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_allgather_kernel(const 
   const int lead = min(a.vshard, (int)((16u - ((uint32_t)reinterpret_cast<uintptr_t>(lg) & 15u)) & 15u) / 4);
   const float4* lv = reinterpret_cast<const float4*>(lg + lead);
   const int nv = (a.vshard - lead) / 4;
-  if ((int)threadIdx.x < lead) better(bv, bi, lg[threadIdx.x], threadIdx.x);
+  if ((int)threadIdx.x < lead) better(bv, bi, lg[threadIdx.x], threadIdx.x, nf);
   for (int i0 = threadIdx.x; i0 < nv; i0 += kVecs * blockDim.x) {
     float4 v[kVecs];
 #pragma unroll
@@ -214,19 +216,19 @@ __global__ void __launch_bounds__(kSampleThreads) sample_allgather_kernel(const 
       const int i = i0 + k * blockDim.x;
       if (i < nv) {
         const int e = lead + 4 * i;
-        better(bv, bi, v[k].x, e);
-        better(bv, bi, v[k].y, e + 1);
-        better(bv, bi, v[k].z, e + 2);
-        better(bv, bi, v[k].w, e + 3);
+        better(bv, bi, v[k].x, e, nf);
+        better(bv, bi, v[k].y, e + 1, nf);
+        better(bv, bi, v[k].z, e + 2, nf);
+        better(bv, bi, v[k].w, e + 3, nf);
       }
     }
   }
-  for (int i = lead + 4 * nv + threadIdx.x; i < a.vshard; i += blockDim.x) better(bv, bi, lg[i], i);
+  for (int i = lead + 4 * nv + threadIdx.x; i < a.vshard; i += blockDim.x) better(bv, bi, lg[i], i, nf);
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) {
     const float ov = __shfl_xor_sync(0xffffffffu, bv, o);
     const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-    better(bv, bi, ov, oi);
+    better(bv, bi, ov, oi, nf);
   }
   if ((threadIdx.x & 31) == 0) {
     s_val[threadIdx.x >> 5] = bv;
@@ -234,7 +236,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_allgather_kernel(const 
   }
   __syncthreads();
   if (threadIdx.x == 0) {
-    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) better(bv, bi, s_val[w], s_idx[w]);
+    for (int w = 1; w < (int)(blockDim.x >> 5); ++w) better(bv, bi, s_val[w], s_idx[w], nf);
     bi += me * a.vshard;
     if (W > 1) {
       const uint32_t flag = sy.epoch + 1;
@@ -272,7 +274,7 @@ __global__ void __launch_bounds__(kSampleThreads) sample_allgather_kernel(const 
     float v = s_val[0];
     int id = s_idx[0];
     for (int p = 1; p < W; ++p)
-      if (s_val[p] > v) {  // ties go to the lowest rank, i.e. the lowest global id
+      if (s_val[p] > v || (nf && s_val[p] != s_val[p] && v == v)) {  // ties go to the lowest rank, i.e. the lowest global id
         v = s_val[p];
         id = s_idx[p];
       }

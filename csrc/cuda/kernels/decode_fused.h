@@ -48,6 +48,7 @@ struct SampleArgs {
   long long* next_tokens = nullptr;  // [rows] global winner
   long long* tokens = nullptr;       // [rows] optional second copy (the next step's input ids)
   int* positions = nullptr;          // [rows] optional, incremented by one
+  int nan_first = 0;                 // 1: a NaN counts as the largest value (the first one wins); 0: NaNs are passed over
 };
 cudaError_t launch_sample_allgather(const RankCtx* ctx, const RankCtx* dev_ctx_table, const SampleArgs* args, int nctx,
                                     cudaStream_t stream);

@@ -147,6 +147,25 @@ def test_sample_allgather(comms, world):
         assert torch.equal(pos[r].cpu(), torch.arange(rows, dtype=torch.int32) + 3)
 
 
+@pytest.mark.parametrize("world", [1, 2, 8])
+@pytest.mark.parametrize("nan_first", [False, True])
+def test_sample_allgather_nan(comms, world, nan_first):
+    """NaNs are passed over, or the first one over all shards wins (torch.max); 33 logits leave a head and a tail around
+    the 16-byte vectors of every second row."""
+    c = comms(world)
+    rows, vs = 6, 33
+    logits = torch.randn(rows, vs * world, generator=torch.Generator().manual_seed(12))
+    logits[1, 5] = logits[1, vs * world - 1] = logits[2, vs - 1] = logits[3, vs * (world - 1)] = float("nan")
+    logits[4, 7], logits[4, 9] = float("inf"), float("nan")
+    shards = [logits[:, r * vs:(r + 1) * vs].contiguous().cuda() for r in range(world)]
+    nxt = [torch.zeros(rows, dtype=torch.int64, device="cuda") for _ in range(world)]
+    c.sample_allgather(shards, nxt, nan_first=nan_first)
+    torch.cuda.synchronize()
+    ref = logits.max(dim=-1).indices if nan_first else logits.nan_to_num(nan=-float("inf"), posinf=float("inf")).argmax(dim=-1)
+    for r in range(world):
+        assert torch.equal(nxt[r].cpu(), ref)
+
+
 def test_abort_word_ends_a_wait_early():
     """abort(): a kernel that waits for a peer that never arrives returns as soon as the host raises the
     communicator's abort word, long before its wait budget, and reports the aborted status."""

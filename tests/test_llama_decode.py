@@ -116,3 +116,20 @@ def test_prefill_fills_every_position_alike(n, S):
     for other in caches[1:]:
         assert all(torch.equal(a, b) for a, b in zip(caches[0], other))
     assert torch.equal(tokens[1], tokens[2])
+
+
+def test_nan_logits_above_the_fused_rows():
+    """Batches that the fused row-parallel kernel does not take sample as torch.max does: the first NaN, a valid id."""
+    from torch_ccl_b200.ops import pack_weight, unpack_weight
+
+    m = _model(batch=70, max_seq=256)
+    assert not m._fused_rows(70)
+    head = unpack_weight(m.lm_head, m.vshard, m.cfg.hidden).clone()
+    for nans in ([37, 900], range(m.vshard)):
+        w = head.clone()
+        w[list(nans)] = float("nan")
+        m.lm_head.copy_(pack_weight(w))
+        m.tokens.copy_(torch.arange(70, device="cuda"))
+        m.positions.zero_()
+        ids = m.decode_step(70)
+        assert (ids == nans[0]).all() and torch.equal(ids, m.logits.max(dim=-1).indices) and torch.equal(m.tokens, ids)

@@ -105,13 +105,14 @@ class _Comm:
         else:
             self.direct.gemm_ar_norm([w_packed], [x], [residual], [weight], [out], eps, splitk)
 
-    def sample(self, logits, next_tokens, tokens, positions):
+    def sample(self, logits, next_tokens, tokens, positions, nan_first=False):
         """Greedy sampling over the vocabulary shards: arg-max, all-gather of the per-rank winners
-        and the bookkeeping for the next step (tokens <- winner, positions += 1) in one kernel."""
+        and the bookkeeping for the next step (tokens <- winner, positions += 1) in one kernel.
+        NaN logits are passed over; with `nan_first` the first one wins, as in torch.max."""
         if self.backend is not None:
-            self.backend.fused_sample_allgather(logits, next_tokens, tokens, positions)
+            self.backend.fused_sample_allgather(logits, next_tokens, tokens, positions, nan_first)
         else:
-            self.direct.sample_allgather([logits], [next_tokens], [tokens], [positions])
+            self.direct.sample_allgather([logits], [next_tokens], [tokens], [positions], nan_first)
 
     def all_reduce(self, t):
         if self.backend is not None:
@@ -265,12 +266,14 @@ class TPLlamaDecoder:
         cfg = self.cfg
         tokens, h, xn = self.tokens[:B], self.h[:B], self.xn[:B]
         self.comm.embed_norm(tokens, self.embed, self.rank * self.vshard, h, self.layers[0]["attn_norm"], xn, cfg.eps)
-        layer = self._layer_fused if self._fused_rows(B) else self._layer_unfused
+        fused_rows = self._fused_rows(B)
+        layer = self._layer_fused if fused_rows else self._layer_unfused
         for li, L in enumerate(self.layers):
             layer(li, B, L["k"], L["v"], self.positions[:B])
         self._gemm_t(self.lm_head, xn, self.logits[:B], self.vshard)
         # feeds the sampled ids back into self.tokens and advances the positions: steady state is a pure replay
-        self.comm.sample(self.logits[:B], self.next_tokens[:B], tokens, self.positions[:B])
+        # (batches above the fused rows choose among NaNs as torch.max does, like the unfused step)
+        self.comm.sample(self.logits[:B], self.next_tokens[:B], tokens, self.positions[:B], nan_first=not fused_rows)
 
     def _decode_body_unfused(self, B):
         cfg = self.cfg
