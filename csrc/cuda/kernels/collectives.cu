@@ -1042,9 +1042,9 @@ __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(const FusedNormAr
   ptx::griddep_launch_dependents();
   const int hv = a.hidden / 8;
   const int row = blockIdx.x;
+  ptx::griddep_wait();  // before the weight too: the kernel before this one may have written it
   Vec<T> wv[MV];
   ll_load_norm_weight<T, MV>(a.weight, 0, hv, wv);
-  ptx::griddep_wait();
   const size_t row_bytes = (size_t)a.hidden * sizeof(T);
   const char* x = static_cast<const char*>(a.x);
   if (a.gather_tokens) {

@@ -206,3 +206,23 @@ def test_full_shard_unit_with_a_sparse_gradient(group):
     want = torch.zeros(40, 16, device="cuda")
     want[3], want[5] = 2.0, 1.0
     assert torch.equal(grad, want)
+
+
+def test_norm_weight_written_by_the_kernel_before(group):
+    """The norm reads its weight after the kernels before it on the stream, which start their successor early."""
+    from torch_ccl_b200 import ops
+
+    rows, hidden, steps = 4, 4096, 50
+    x = torch.randn(rows, hidden, device="cuda").bfloat16()
+    n = (x.float() * torch.rsqrt(x.float().pow(2).mean(-1, keepdim=True) + 1e-5)).bfloat16()
+    # the cast is long (its tail is the weight), so that an early read would find the weight of the step before
+    long_in = [torch.full((1 << 24,), float(i), device="cuda").bfloat16() for i in (1, 2)]
+    long_out = torch.zeros(1 << 24, device="cuda").bfloat16()
+    w = long_out[-hidden:]
+    res = torch.zeros(steps, rows, hidden, device="cuda").bfloat16()
+    got = []
+    for i in range(steps):  # (nothing of torch's between the two, which would wait for the first)
+        ops.reduce_scatter_cast(long_in[i % 2], long_out)
+        got.append(ops.allreduce_residual_rmsnorm(x, res[i], w))
+    for i, y in enumerate(got):
+        torch.testing.assert_close(y.float(), n.float() * (1 + i % 2), rtol=2.0**-7, atol=1e-6)
