@@ -554,13 +554,23 @@ cudaError_t CudaComm::plain_gemm(const void* a, const void* b, void* out, int64_
   return e;
 }
 
+namespace {
+// Memory of a rows x cols bf16 matrix with row stride ld.
+bool overlap(const void* p, int64_t prows, int64_t pcols, int64_t pld, const void* q, int64_t qrows, int64_t qcols, int64_t qld) {
+  const uintptr_t a = reinterpret_cast<uintptr_t>(p), b = reinterpret_cast<uintptr_t>(q);
+  return a < b + 2 * ((qrows - 1) * qld + qcols) && b < a + 2 * ((prows - 1) * pld + pcols);
+}
+}  // namespace
+
 cudaError_t CudaComm::gemm_rs(const std::vector<GemmRsArgs>& args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
   enter_stream(stream);
-  if (world_ == 1) {
+  const GemmRsArgs& a = args[0];
+  // A result that shares memory with an operand is staged also when there is nobody to exchange with: the plain kernel would
+  // store tiles while others still read.
+  if (world_ == 1 && !overlap(a.out, a.M, a.N, a.N, a.a, a.M, a.K, a.lda) && !overlap(a.out, a.M, a.N, a.N, a.b, a.N, a.K, a.ldb)) {
     // nobody to exchange with: the plain kernel straight into the result (no staging, no reduce pass)
-    const GemmRsArgs& a = args[0];
     if (a.M % 128 != 0 || a.N % 16 != 0 || a.K % 8 != 0) return cudaErrorInvalidValue;
     return plain_gemm(a.a, a.b, a.out, a.M, a.N, a.K, a.lda, a.ldb, a.N, stream);
   }

@@ -153,6 +153,25 @@ def test_gemm_collective_ops_alone(comm, M, N, K):
         assert ((out.float() - ref).norm() / ref.norm()).item() <= 2.0**-9 + K * 2.0**-24
 
 
+@pytest.mark.parametrize("M,K", [(256, 1024), (1024, 256)])
+def test_gemm_rs_result_over_an_operand(comm, M, K):
+    """out= may share memory with either operand (N = K, or N = K = M)."""
+    g = torch.Generator(device="cuda").manual_seed(M)
+    a, b = torch.randn(M, K, generator=g, device="cuda").bfloat16(), torch.randn(K, K, generator=g, device="cuda").bfloat16()
+    want = torch.empty(M, K, device="cuda", dtype=torch.bfloat16)
+    comm.gemm_rs([a], [b], [want])
+    for shift in (0, 3):  # the same rows, and rows further on in one allocation
+        both = torch.zeros(M + shift, K, device="cuda", dtype=torch.bfloat16)
+        both[shift:] = a
+        comm.gemm_rs([both[shift:]], [b], [both[:M]])
+        assert torch.equal(both[:M], want)
+    if M >= K:
+        over = torch.zeros(M, K, device="cuda", dtype=torch.bfloat16)
+        over[:K] = b
+        comm.gemm_rs([a], [over[:K]], [over])
+        assert torch.equal(over, want)
+
+
 @pytest.fixture()
 def group():
     import torch.distributed as dist
