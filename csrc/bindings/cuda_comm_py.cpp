@@ -40,6 +40,12 @@ ccl::KvStore make_kv(const c10::intrusive_ptr<c10d::Store>& store) {
   return kv;
 }
 
+// Whether two contiguous tensors share memory.
+static bool share(const at::Tensor& a, const at::Tensor& b) {
+  const char *p = static_cast<const char*>(a.data_ptr()), *q = static_cast<const char*>(b.data_ptr());
+  return p < q + b.nbytes() && q < p + a.nbytes();
+}
+
 void fill_moe_dispatch(ccl::MoeArgs& a, const at::Tensor& x, const at::Tensor& idx, at::Tensor& out_x, at::Tensor& meta,
                        at::Tensor& count, int experts_per_rank) {
   TORCH_CHECK(x.scalar_type() == at::kBFloat16 && x.is_contiguous() && x.dim() == 2, "x: [tokens, hidden] bf16");
@@ -57,6 +63,7 @@ void fill_moe_dispatch(ccl::MoeArgs& a, const at::Tensor& x, const at::Tensor& i
   a.hidden = (int)x.size(1);
   a.experts_per_rank = experts_per_rank;
   a.max_rows = (int)out_x.size(0);
+  for (const at::Tensor* out : {&out_x, &meta, &count}) a.staged |= share(*out, x) || share(*out, idx);
 }
 
 void fill_moe_combine(ccl::MoeArgs& a, const at::Tensor& y, const at::Tensor& meta, const at::Tensor& count,
@@ -72,6 +79,7 @@ void fill_moe_combine(ccl::MoeArgs& a, const at::Tensor& y, const at::Tensor& me
   a.tokens = (int)gate.size(0);
   a.topk = (int)gate.size(1);
   a.hidden = (int)y.size(1);
+  a.staged = share(out, y) || share(out, meta) || share(out, count);
 }
 
 ccl::FusedNormArgs make_norm_args(const at::Tensor& x, at::Tensor& residual, const at::Tensor& weight, at::Tensor& out, double eps,

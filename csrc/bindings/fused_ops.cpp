@@ -199,11 +199,11 @@ void moe_dispatch(ProcessGroupCCL& pg, const at::Tensor& x, const at::Tensor& id
   auto& c = cuda_comm_of(pg, x);
   c10::cuda::CUDAGuard g(x.device());
   ccl::MoeArgs a;
+  ccl_py::fill_moe_dispatch(a, x, idx, out_x, meta, count, (int)experts_per_rank);
   if (clear_count) {
-    if (c.world() == 1) a.count_len = (int)count.numel();
+    if (c.world() == 1 && !a.staged) a.count_len = (int)count.numel();
     else count.zero_();
   }
-  ccl_py::fill_moe_dispatch(a, x, idx, out_x, meta, count, (int)experts_per_rank);
   C10_CUDA_CHECK(c.moe_dispatch({a}, c10::cuda::getCurrentCUDAStream()));
 }
 

@@ -372,8 +372,12 @@ size_t moe_dispatch_slot_bytes(int cap, int hidden) {
   return round_up((size_t)cap * hidden * 2 + (size_t)cap * 8 + (size_t)kMaxBlocks * 4, 256);
 }
 
+// The local kernels write results while other CTAs still read, so a call whose results share memory with its inputs keeps
+// the staged form, which writes after every read.
 cudaError_t launch_moe_dispatch(const RankCtx* ctx, const MoeArgs* args, const LaunchCfg& cfg) {
-  if (!cfg.cooperative && ctx->world == 1) {
+  if (!cfg.cooperative && ctx->world == 1 && args->staged && args->tokens * args->topk > args->max_rows)
+    return cudaErrorInvalidValue;  // that form does not look at what out_x holds
+  if (!cfg.cooperative && ctx->world == 1 && !args->staged) {
     int threads = 0;
     const dim3 grid = local_grid(*args, &threads);
     return launch_local(moe_dispatch_local_kernel, grid, threads, cfg.stream, *args, ctx->status);
@@ -381,7 +385,7 @@ cudaError_t launch_moe_dispatch(const RankCtx* ctx, const MoeArgs* args, const L
   return launch_moe(moe_dispatch_kernel<false>, moe_dispatch_kernel<true>, ctx, args, cfg);
 }
 cudaError_t launch_moe_combine(const RankCtx* ctx, const MoeArgs* args, const LaunchCfg& cfg) {
-  if (!cfg.cooperative && ctx->world == 1) {
+  if (!cfg.cooperative && ctx->world == 1 && !args->staged) {
     // the inverse (a word per slot) lives in the arena, which nothing else of a one-rank communicator uses
     int* inverse = reinterpret_cast<int*>(ctx->data[0]);
     const int slots = args->tokens * args->topk;

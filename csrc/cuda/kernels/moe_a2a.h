@@ -23,6 +23,7 @@ struct MoeArgs {
   unsigned long long slot_bytes = 0;  // moe_dispatch_slot_bytes(cap, hidden)
   int max_rows = 0;                 // dispatch: rows that out_x holds
   int count_len = 0;                // dispatch: words of out_count to define (0: only those listed above)
+  int staged = 0;                   // a result shares memory with an input: through the arena also with one rank
 };
 
 size_t moe_dispatch_slot_bytes(int cap, int hidden);

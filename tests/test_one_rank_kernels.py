@@ -113,6 +113,33 @@ def test_moe(comm, tokens, hidden, experts, topk):
         assert ((out.double() - ref).abs() <= bound + ref.abs() * 2.0**-8).all()
 
 
+@pytest.mark.parametrize("shift", [0, 5])
+def test_moe_results_over_inputs(comm, shift):
+    """out= of combine may share memory with the rows that it sums (one expert a token), and dispatch's rows with x."""
+    T, H = 300, 512
+    g = torch.Generator(device="cuda").manual_seed(shift)
+    store = torch.zeros(T + shift, H, device="cuda", dtype=torch.bfloat16)
+    y, out = store[shift:], store[:T]
+    y.copy_(torch.randn(T, H, generator=g, device="cuda"))
+    src = y.clone()
+    gate = torch.rand(T, 1, generator=g, device="cuda")
+    slot = torch.randperm(T, generator=g, device="cuda").int()
+    meta = torch.stack([torch.zeros_like(slot), slot, torch.zeros_like(slot)], 1).contiguous()
+    count = torch.zeros(16, device="cuda", dtype=torch.int32)
+    count[:2] = T
+    comm.moe_combine([y], [meta], [count], [gate], [out])
+    want = torch.empty_like(src)
+    want[slot.long()] = src
+    assert torch.equal(out, (want.float() * gate).bfloat16())
+
+    y.copy_(src)
+    idx = torch.zeros(T, 1, device="cuda", dtype=torch.int32)
+    comm.moe_dispatch([y], [idx], [out], [meta], [count], 1)
+    assert torch.equal(out, src[meta[:, 1].long()]) and sorted(meta[:, 1].tolist()) == list(range(T)) and int(count[0]) == T
+    with pytest.raises(RuntimeError, match="moe_dispatch"):
+        comm.moe_dispatch([y], [idx], [out[: T - 1]], [meta], [count], 1)
+
+
 def test_moe_over_capacity(comm):
     """Rows that out_x has no room for are dropped and reported."""
     x, idx = torch.ones(4, 64, device="cuda").bfloat16(), torch.zeros(4, 2, device="cuda", dtype=torch.int32)
