@@ -1,5 +1,6 @@
 #include "bindings/fused_ops.h"
 
+#include <ATen/MemoryOverlap.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 
@@ -89,7 +90,10 @@ void reduce_scatter_cast(ProcessGroupCCL& pg, const at::Tensor& inp, at::Tensor&
     a.scale = (float)scale;
   }
   if (W == 1) {
-    if (at::isFloatingType(inp.scalar_type()) && inp.scalar_type() != at::kDouble) {
+    // in place, and for the types that the kernel does not have, torch's own copy and scale
+    const auto st = inp.scalar_type();
+    at::assert_no_partial_overlap(out, inp);
+    if ((st == at::kBFloat16 || st == at::kHalf || st == at::kFloat) && inp.data_ptr() != out.data_ptr()) {
       ccl::CastTable t;
       t.src[0] = inp.data_ptr();
       t.off[0] = 0;
@@ -97,7 +101,7 @@ void reduce_scatter_cast(ProcessGroupCCL& pg, const at::Tensor& inp, at::Tensor&
       t.n = 1;
       t.dst = out.data_ptr();
       t.scale = (float)scale;
-      C10_CUDA_CHECK(ccl::launch_cast_table(to_ccl_dtype(inp.scalar_type()), to_ccl_dtype(out.scalar_type()), false, t, c10::cuda::getCurrentCUDAStream()));
+      C10_CUDA_CHECK(ccl::launch_cast_table(to_ccl_dtype(st), to_ccl_dtype(out.scalar_type()), false, t, c10::cuda::getCurrentCUDAStream()));
       return;
     }
     out.copy_(inp.view_as(out));

@@ -272,3 +272,20 @@ def test_norm_weight_written_by_the_kernel_before(group):
         got.append(ops.allreduce_residual_rmsnorm(x, res[i], w))
     for i, y in enumerate(got):
         torch.testing.assert_close(y.float(), n.float() * (1 + i % 2), rtol=2.0**-7, atol=1e-6)
+
+
+def test_reduce_scatter_cast_types_and_overlap(group):
+    """With one rank: every type that torch copies, in place, and no partial overlap."""
+    from torch_ccl_b200 import ops
+
+    x = torch.randn(1000, device="cuda")
+    for dt in (torch.float32, torch.float16, torch.bfloat16, torch.float64, torch.float8_e4m3fn, torch.int32):
+        a = (x * 10).to(dt)
+        for out_dt in {dt, torch.float32}:
+            out = torch.empty(1000, device="cuda", dtype=out_dt)
+            assert torch.equal(ops.reduce_scatter_cast(a, out).float(), a.float())
+    own = x.clone()
+    assert torch.equal(ops.reduce_scatter_cast(own, own, 0.5), x * 0.5)
+    for a, out in ((own[:500], own[100:600]), (own.view(torch.bfloat16)[:500], own[:500])):
+        with pytest.raises(RuntimeError, match="memory location"):
+            ops.reduce_scatter_cast(a, out)
