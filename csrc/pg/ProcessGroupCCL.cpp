@@ -136,6 +136,7 @@ c10::intrusive_ptr<c10::ivalue::Future> ProcessGroupCCL::AsyncWorkCCL::getFuture
     makeFuture(nested_, devs);
     if (done_err_) future_->setError(done_err_);
     else if (done_ok_ || !devs.empty()) completeFutureNow();  // CUDA work: stream-ordered completion
+    else self_ = c10::intrusive_ptr<AsyncWorkCCL>::reclaim_copy(this);
   }
   return future_;
 }
@@ -149,8 +150,10 @@ std::vector<at::Tensor> ProcessGroupCCL::AsyncWorkCCL::result() {
 }
 
 void ProcessGroupCCL::AsyncWorkCCL::finishOk() {
+  c10::intrusive_ptr<AsyncWorkCCL> self;  // let go after the last use of this
   {
     std::lock_guard<std::mutex> g(fut_mu_);
+    self = std::move(self_);
     done_ok_ = true;
     if (future_ && !future_->completed()) completeFutureNow();
   }
@@ -169,8 +172,10 @@ bool ProcessGroupCCL::AsyncWorkCCL::wait(std::chrono::milliseconds timeout) {
 }
 
 void ProcessGroupCCL::AsyncWorkCCL::finishError(std::exception_ptr e) {
+  c10::intrusive_ptr<AsyncWorkCCL> self;
   {
     std::lock_guard<std::mutex> g(fut_mu_);
+    self = std::move(self_);
     done_err_ = e;
     if (future_ && !future_->completed()) future_->setError(e);
   }

@@ -79,6 +79,9 @@ class ProcessGroupCCL : public Backend {
     bool done_ok_ = false;
     std::exception_ptr done_err_;
     c10::intrusive_ptr<c10::ivalue::Future> future_;
+    // Set from the hand-out of an incomplete future until the work ends: whoever completes works may know this one weakly, and
+    // the future has to be completed also when its holder has let the work go.
+    c10::intrusive_ptr<AsyncWorkCCL> self_;
     std::vector<at::Tensor> outputs_;
     std::vector<std::vector<at::Tensor>> nested_outputs_;
     bool nested_ = false;

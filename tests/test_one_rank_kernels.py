@@ -289,3 +289,22 @@ def test_reduce_scatter_cast_types_and_overlap(group):
     for a, out in ((own[:500], own[100:600]), (own.view(torch.bfloat16)[:500], own[:500])):
         with pytest.raises(RuntimeError, match="memory location"):
             ops.reduce_scatter_cast(a, out)
+
+
+@pytest.mark.parametrize("pending", [False, True])
+def test_future_of_a_dropped_work(group, pending):
+    """A future without tensors is completed, and its callbacks run, also when its holder has let the Work go."""
+    import time
+
+    import torch.distributed as dist
+
+    dist.barrier(device_ids=[0])  # set-up of the communicator
+    if pending:
+        torch.cuda._sleep(100_000_000)
+    fut = dist.barrier(async_op=True, device_ids=[0]).get_future()
+    called = []
+    fut.add_done_callback(lambda f: called.append(1))
+    limit = time.time() + 10
+    while not (fut.done() and called) and time.time() < limit:
+        time.sleep(0.001)
+    assert fut.done() and called == [1]
