@@ -52,8 +52,7 @@ struct Desc2 {
 };
 
 // Tile width for the CTA-pair kernel.
-int pick_bn(int64_t M, int64_t N, int64_t K, bool dual, bool packed) {
-  (void)K;
+int pick_bn(int64_t M, int64_t N, bool dual, bool packed) {
   const int64_t mt = (M + 2 * kBM - 1) / (2 * kBM);
   double best = 1e30;
   int bn = 256;
@@ -144,7 +143,7 @@ cudaError_t dispatch_2sm(const GemmDesc& d, cudaStream_t stream) {
     q.ldb = d.ldb;
   }
   // a given width counts result columns (dual: of each half)
-  int bn = d.bn > 0 ? std::min(256, d.dual_off > 0 ? 2 * d.bn : d.bn) : pick_bn(q.M, q.N, q.K, d.dual_off > 0, q.b_tiled != 0);
+  int bn = d.bn > 0 ? std::min(256, d.dual_off > 0 ? 2 * d.bn : d.bn) : pick_bn(q.M, q.N, d.dual_off > 0, q.b_tiled != 0);
   if (d.dual_off > 0) return d.out_fp32 ? launch_2sm<true, float>(d, q, bn, stream) : launch_2sm<true, __nv_bfloat16>(d, q, bn, stream);
   return d.out_fp32 ? launch_2sm<false, float>(d, q, bn, stream) : launch_2sm<false, __nv_bfloat16>(d, q, bn, stream);
 }
@@ -257,11 +256,15 @@ cudaError_t gemm_bf16_tn(const GemmDesc& d, cudaStream_t stream) {
   if ((reinterpret_cast<uintptr_t>(d.a) & 15) || (reinterpret_cast<uintptr_t>(d.b) & 15))
     return cudaErrorInvalidValue;
   // Many result rows: the CTA-pair kernel, whose result is row-major (with trans_out the rows are B's; a dual or packed A
-  // can only be its B operand, so those need trans_out).
+  // can only be its B operand, so those need trans_out). Up to 64 columns the one-CTA kernel below stays the better one: it
+  // streams A through narrow tiles and splits K (us, pairs / one CTA, at K = 4096 and 16384: 256 x 16 20.5 / 10.2 and 57.3 /
+  // 14.3, 4096 x 16 24.6 / 16.4 and 69.6 / 36.9, 1024 x 64 22.5 / 16.4 and 59.4 / 34.8); from 65 on it has no split and took
+  // 32.8 and 102.4 for 256 x 80 where pairs take 20.5 and 57.3.
   if (d.a_tiled && d.dual_off % gemm::kBM != 0) return cudaErrorInvalidValue;  // gate and up start on whole packed tiles
   const bool width_ok = d.bn == 0 || d.bn == 64 || d.bn == 128 || (d.bn == 256 && d.dual_off == 0) ||
                         (d.bn > 64 && d.bn < 256 && d.bn % 32 == 0 && !d.a_tiled && d.dual_off == 0);
-  if (width_ok && d.splitk <= 1 && (d.trans_out ? d.N : d.M) > 128 && (d.trans_out || (!d.a_tiled && d.dual_off == 0)))
+  if (width_ok && d.splitk <= 1 && (d.trans_out ? d.N : d.M) > 128 &&
+      (d.trans_out || (!d.a_tiled && d.dual_off == 0 && d.N > 64)))
     return gemm::dispatch_2sm(d, stream);
   int bn = d.bn;
   if (bn == 0) {

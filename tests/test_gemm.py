@@ -159,3 +159,17 @@ def test_gemm_cta_pairs_packed(rows, K, tokens, dual):
         ref = _ref(x, w[0])
     torch.cuda.synchronize()
     assert ((out.float() - ref).norm() / ref.norm()).item() <= 2.0**-9 + K * 2.0**-22  # silu's __expf adds 2 ulp
+
+
+@pytest.mark.parametrize("M,N,K,width,split", [(256, 32, 16384, 32, 16), (4096, 16, 8192, 16, 8), (300, 64, 4096, 64, 4), (130, 17, 64, 32, 1)])
+def test_gemm_narrow_results_split_k(M, N, K, width, split):
+    """More than 128 rows but at most 64 columns: narrow tiles, K split over a cluster (the sums say which kernel it was)."""
+    torch.manual_seed(8)
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    auto, given = (torch.empty(M, N, device="cuda") for _ in range(2))
+    _C().gemm_bf16_tn(a, b, auto)
+    _C().gemm_bf16_tn(a, b, given, False, 0, split, width)
+    assert torch.equal(auto, given)
+    ref = _ref(a, b)
+    assert ((auto - ref).norm() / ref.norm()).item() <= K * 2.0**-24
