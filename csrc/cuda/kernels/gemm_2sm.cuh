@@ -145,6 +145,7 @@ __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
     }
   } else if (warp == 1) {
     if (rank == 0 && ptx::elect_one()) {
+      ptx::griddep_wait();  // the first operands come after it: the time limits of the waits below start here
       const uint32_t idesc = ptx::make_idesc_bf16(2 * kBM, p.bn);
       // the loop below is one thread's serial chain: no divisions, and the descriptors only by addition
       const uint64_t desc_a0 = ptx::make_desc_sw128(ptx::smem_u32(smem));

@@ -265,6 +265,7 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap* tma_a, const C
     }
   } else if (warp == 1) {
     if (ptx::elect_one()) {
+      ptx::griddep_wait();  // B comes after it: the time limits of the waits below start here
       constexpr uint32_t idesc = ptx::make_idesc_bf16(kBM, BN);
       const uint64_t desc_a0 = ptx::make_desc_sw128(ptx::smem_u32(smem));
       int s = 0;
@@ -296,16 +297,15 @@ __device__ __forceinline__ void gemm_tile_body(const CUtensorMap* tma_a, const C
     // ---- epilogue warps -------------------------------------------------------------------
     const int q = warp & 3;
     const int row = q * 32 + lane;
+    // the accumulator comes after the predecessor grid, and so do the time limit of the wait for it and whatever these
+    // threads read or overwrite from an earlier kernel
+    ptx::griddep_wait();
     bool ok = ptx::mbar_wait(&bars->accum, 0);
     if (!ok) {
       bars->failed = 1;
       if (p.status) atomicExch(p.status, 103);
     }
     ptx::tc_fence_after();
-    // the producer already waited for the predecessor grid before it fetched B; the epilogue
-    // threads repeat the (by now satisfied) wait so that whatever they read or overwrite from an
-    // earlier kernel is ordered for them too
-    ptx::griddep_wait();
     if (p.splitk > 1) {
       // reduce-scatter: send this row's partial to the CTA that owns the row
       // (buffer layout at the owner: [source slot][column group of 4][local row] float4)

@@ -173,3 +173,23 @@ def test_gemm_narrow_results_split_k(M, N, K, width, split):
     assert torch.equal(auto, given)
     ref = _ref(a, b)
     assert ((auto - ref).norm() / ref.norm()).item() <= K * 2.0**-24
+
+
+@pytest.mark.parametrize("M,N,K", [(300, 128, 256), (16, 128, 256), (300, 16, 1024)])
+def test_gemm_behind_a_late_kernel(M, N, K):
+    """A GEMM starts early and waits for the kernel before it, which may itself wait for a peer for longer than the GEMM's own
+    waits are allowed to take (here: two and a half seconds, for a peer that does not exist)."""
+    C = _C()
+    c = C.CudaComm.emulated(2, 1 << 20, 2500, 1)
+    a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
+    b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
+    out = torch.empty(M, N, device="cuda")
+    C.gemm_bf16_tn(a, b, out)
+    want = out.clone()
+    out.fill_(float("nan"))
+    torch.cuda.synchronize()
+    C.emu_missing_peer_probe(c)
+    C.gemm_bf16_tn(a, b, out)
+    torch.cuda.synchronize()
+    assert c.status()[0] == 1
+    assert torch.equal(out, want)
