@@ -176,18 +176,24 @@ void CudaComm::clear_status() {
 
 // One launch in flight per communicator: the kernels of a communicator share its epoch, ticket and
 // staging halves, so two of them must never run concurrently. Launches on one stream are ordered
-// by the stream; when the caller moves to another stream (c10d ops run on the backend's
-// communication stream, the fused ops on the caller's current stream) the new stream is made to
-// wait for everything enqueued on the previous one. Costs nothing while the stream stays the
-// same. Streams that are being captured are left alone: inside a CUDA graph the capture's own
-// dependencies order the launches.
-void CudaComm::enter_stream(cudaStream_t s) {
-  std::lock_guard<std::mutex> g(order_mu_);
+// by the stream; when the caller moves to another stream (asynchronous c10d ops run on the backend's
+// communication stream, the others and the fused ops on the caller's current stream) the new stream is
+// made to wait for everything enqueued on the previous one. Costs nothing while the stream stays the
+// same. The lock is kept until the caller has enqueued its kernels: another thread's launch on
+// another stream then finds them in front of the event that it waits for. Streams of one capture are
+// ordered by an edge of its graph; between a captured and an eager launch there is no order to record
+// (that is the order in which the program replays the graph).
+static bool capture_of(cudaStream_t s, unsigned long long* id) {
+  cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+  *id = 0;
+  return cudaStreamGetCaptureInfo(s, &st, id) == cudaSuccess && (st == cudaStreamCaptureStatusActive || st == cudaStreamCaptureStatusNone);
+}
+
+std::unique_lock<std::recursive_mutex> CudaComm::enter_stream(cudaStream_t s) {
+  std::unique_lock<std::recursive_mutex> lock(order_mu_);
   if (has_last_stream_ && last_stream_ != s) {
-    cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone, cl = cudaStreamCaptureStatusNone;
-    const bool q = cudaStreamIsCapturing(s, &cs) == cudaSuccess && cudaStreamIsCapturing(last_stream_, &cl) == cudaSuccess;
-    if (q && cs == cudaStreamCaptureStatusNone && cl == cudaStreamCaptureStatusNone &&
-        cudaEventRecord(order_ev_, last_stream_) == cudaSuccess) {
+    unsigned long long now = 0, before = 0;
+    if (capture_of(s, &now) && capture_of(last_stream_, &before) && now == before && cudaEventRecord(order_ev_, last_stream_) == cudaSuccess) {
       cudaStreamWaitEvent(s, order_ev_, 0);
     } else {
       (void)cudaGetLastError();
@@ -195,6 +201,7 @@ void CudaComm::enter_stream(cudaStream_t s) {
   }
   last_stream_ = s;
   has_last_stream_ = true;
+  return lock;
 }
 
 template <typename ArgsT>
@@ -263,7 +270,7 @@ static size_t cap_stride(size_t stride, size_t slots, size_t round_bytes) {
 cudaError_t CudaComm::allreduce(int dtype, std::vector<CollArgs> args, cudaStream_t stream, AlgoChoice* chosen) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   const size_t esz = dtype_size(dtype);
   const size_t count = args[0].count;
   const size_t bytes = count * esz;
@@ -327,7 +334,7 @@ cudaError_t CudaComm::allreduce(int dtype, std::vector<CollArgs> args, cudaStrea
 cudaError_t CudaComm::reduce(int dtype, std::vector<CollArgs> args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   const size_t nvec = (args[0].count * dtype_size(dtype) + 15) / 16;
   size_t stride = cfg_.half_bytes / (16 * (size_t)(world_ + 1));
   stride = compact_stride(stride / 8 * 8, (nvec + world_ - 1) / world_);
@@ -344,7 +351,7 @@ cudaError_t CudaComm::reduce(int dtype, std::vector<CollArgs> args, cudaStream_t
 cudaError_t CudaComm::reduce_scatter(int in_dtype, int out_dtype, std::vector<CollArgs> args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   const size_t esz = dtype_size(in_dtype);
   // flat symmetric input (equal pieces, back to back, inside the heap): reduce straight out of the peers' buffers
   if (world_ > 1 && !heap_bases_.empty() && cfg_.ablate == kAblateNone && (cfg_.algo == Algo::kAuto || cfg_.algo == Algo::kNvls)) {
@@ -397,7 +404,7 @@ cudaError_t CudaComm::reduce_scatter(int in_dtype, int out_dtype, std::vector<Co
 cudaError_t CudaComm::all_gather(std::vector<CollArgs> args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   // flat symmetric output (equal pieces, back to back, inside the heap): write straight into the peers' buffers
   if (world_ > 1 && !heap_bases_.empty() && cfg_.ablate == kAblateNone && (cfg_.algo == Algo::kAuto || cfg_.algo == Algo::kNvls)) {
     const size_t pb = args[0].out_cnt[0];
@@ -451,7 +458,7 @@ cudaError_t CudaComm::all_gather(std::vector<CollArgs> args, cudaStream_t stream
 cudaError_t CudaComm::all_to_all(std::vector<CollArgs> args, bool uneven, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   // the round cap pays for up to four ranks (512 MB: 680 -> 643 us at 2, 819 -> 798 at 4); at eight it does not (920 -> 948)
   size_t stride = cap_stride(cfg_.half_bytes / (16 * (size_t)world_), world_, (uneven || world_ > 4) ? 0 : cfg_.round_bytes);
   stride = stride / 8 * 8;
@@ -478,7 +485,7 @@ cudaError_t CudaComm::all_to_all(std::vector<CollArgs> args, bool uneven, cudaSt
 cudaError_t CudaComm::rooted(std::vector<CollArgs> args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   int mode = args[0].mode;
   if (mode == kBroadcast && world_ > 1 && cfg_.ablate == kAblateNone) {
     // Large broadcasts leave the root once and are replicated by the switch.
@@ -515,7 +522,7 @@ bool CudaComm::multi_fits(int dtype, const MultiArgs& a) const {
 cudaError_t CudaComm::multi(int dtype, std::vector<MultiArgs> args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   if (!multi_fits(dtype, args[0])) return cudaErrorInvalidValue;
   const size_t slot = multi_slot_bytes(dtype, args[0]);
   for (auto& a : args) a.slot_bytes = slot;
@@ -528,7 +535,7 @@ cudaError_t CudaComm::multi(int dtype, std::vector<MultiArgs> args, cudaStream_t
 
 cudaError_t CudaComm::barrier(cudaStream_t stream) {
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   std::vector<CollArgs> args(nctx());
   for (auto& a : args) a.ablate = kAblateNone;
   LaunchCfg lc = launch_cfg(1, 32, stream);
@@ -565,7 +572,7 @@ bool overlap(const void* p, int64_t prows, int64_t pcols, int64_t pld, const voi
 cudaError_t CudaComm::gemm_rs(const std::vector<GemmRsArgs>& args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   const GemmRsArgs& a = args[0];
   // A result that shares memory with an operand is staged also when there is nobody to exchange with: the plain kernel would
   // store tiles while others still read.
@@ -593,7 +600,7 @@ cudaError_t CudaComm::gemm_rs(const std::vector<GemmRsArgs>& args, cudaStream_t 
 cudaError_t CudaComm::ag_gemm(const std::vector<AgGemmArgs>& args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   const int ncomm = 8;
   if (world_ == 1) {
     const AgGemmArgs& a = args[0];
@@ -625,7 +632,7 @@ int CudaComm::moe_capacity(int hidden) const {
 cudaError_t CudaComm::moe_dispatch(std::vector<MoeArgs> args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   const int cap = moe_capacity(args[0].hidden);
   if (cap <= 0 || args[0].hidden % 8 != 0) return cudaErrorInvalidValue;
   for (auto& a : args) {
@@ -645,7 +652,7 @@ cudaError_t CudaComm::moe_dispatch(std::vector<MoeArgs> args, cudaStream_t strea
 cudaError_t CudaComm::moe_combine(std::vector<MoeArgs> args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   if ((size_t)args[0].tokens * args[0].topk * args[0].hidden * 2 > cfg_.half_bytes) return cudaErrorInvalidValue;
   LaunchCfg lc = launch_cfg(std::min(64, cfg_.max_blocks), 512, stream);
   cudaError_t e = launch_moe_combine(emulated_ ? dev_ctx_table_ : host_ctx_.data(), upload(args, stream), lc);
@@ -655,7 +662,7 @@ cudaError_t CudaComm::moe_combine(std::vector<MoeArgs> args, cudaStream_t stream
 
 cudaError_t CudaComm::barrier_single_rank(int i, cudaStream_t stream) {
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   if (i < 0 || i >= nctx()) return cudaErrorInvalidValue;
   CollArgs a;
   LaunchCfg lc;
@@ -757,7 +764,7 @@ static bool switch_dtype(int dt) { return dt == kBF16 || dt == kF16 || dt == kF3
 cudaError_t CudaComm::allreduce_symm(int dtype, size_t in_off, size_t out_off, size_t count, int op, float scale, int has_scale,
                                      bool use_nvls, cudaStream_t stream) {
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   const size_t bytes = count * dtype_size(dtype);
   if (bytes % 16 || in_off % 16 || out_off % 16 || heap_bases_.empty()) return cudaErrorInvalidValue;
   std::vector<SymmArgs> args(nctx());
@@ -782,7 +789,7 @@ cudaError_t CudaComm::reduce_scatter_symm(int in_dtype, int out_dtype, size_t in
                                           float scale, int has_scale, bool use_nvls, cudaStream_t stream) {
   CCL_CHECK_ARGS(outs)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   const size_t bytes = count * dtype_size(in_dtype);
   if (bytes % 16 || in_off % 16 || heap_bases_.empty()) return cudaErrorInvalidValue;
   std::vector<SymmArgs> args(nctx());
@@ -807,7 +814,7 @@ cudaError_t CudaComm::reduce_scatter_symm(int in_dtype, int out_dtype, size_t in
 cudaError_t CudaComm::all_gather_symm(std::vector<const void*> ins, size_t out_off, size_t bytes, bool use_nvls, cudaStream_t stream) {
   CCL_CHECK_ARGS(ins)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   if (bytes % 16 || out_off % 16 || heap_bases_.empty()) return cudaErrorInvalidValue;
   std::vector<SymmArgs> args(nctx());
   for (int i = 0; i < nctx(); ++i) {
@@ -847,7 +854,7 @@ bool CudaComm::fits_gemm_ar_norm(int rows, int hidden, int K) const {
 cudaError_t CudaComm::gemm_ar_norm(const std::vector<GemmArNormArgs>& args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   cudaError_t e = launch_gemm_ar_norm(host_ctx_.data(), dev_ctx_table_, args.data(), nctx(), stream);
   if (e == cudaSuccess) ++launches_;
   return e;
@@ -856,7 +863,7 @@ cudaError_t CudaComm::gemm_ar_norm(const std::vector<GemmArNormArgs>& args, cuda
 cudaError_t CudaComm::sample_allgather(const std::vector<SampleArgs>& args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   cudaError_t e = launch_sample_allgather(host_ctx_.data(), dev_ctx_table_, args.data(), nctx(), stream);
   if (e == cudaSuccess) ++launches_;
   return e;
@@ -865,7 +872,7 @@ cudaError_t CudaComm::sample_allgather(const std::vector<SampleArgs>& args, cuda
 cudaError_t CudaComm::allreduce_residual_rmsnorm(int dtype, std::vector<FusedNormArgs> args, cudaStream_t stream) {
   CCL_CHECK_ARGS(args)
   DeviceGuard g(device_);
-  enter_stream(stream);
+  const auto order = enter_stream(stream);
   const FusedNormArgs& a0 = args[0];
   if (a0.hidden % 8 != 0 || a0.rows <= 0) return cudaErrorInvalidValue;
   int threads = std::min(512, std::max(32, ((a0.hidden / 8 + 31) / 32) * 32));  // kernel is compiled for <= 512 threads

@@ -182,7 +182,7 @@ class CudaComm {
   void init_tables();
   cudaError_t plain_gemm(const void* a, const void* b, void* out, int64_t M, int64_t N, int64_t K, int64_t lda, int64_t ldb, int64_t ldo,
                          cudaStream_t stream);
-  void enter_stream(cudaStream_t s);
+  std::unique_lock<std::recursive_mutex> enter_stream(cudaStream_t s);  // keep until the kernels are enqueued
   template <typename ArgsT>
   const ArgsT* upload(const std::vector<ArgsT>& args, cudaStream_t stream);
   LaunchCfg launch_cfg(int nblocks, int nthreads, cudaStream_t stream) const;
@@ -210,7 +210,7 @@ class CudaComm {
   mutable std::mutex heap_mu_;
   std::vector<std::pair<size_t, size_t>> heap_free_;   // sorted (offset, size) holes
   std::vector<std::pair<size_t, size_t>> heap_used_;   // (offset, size) of live blocks
-  std::mutex order_mu_;
+  std::recursive_mutex order_mu_;     // (an op may be made of others)
   cudaEvent_t order_ev_ = nullptr;
   cudaStream_t last_stream_ = nullptr;
   bool has_last_stream_ = false;

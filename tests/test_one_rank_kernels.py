@@ -140,6 +140,53 @@ def test_moe_results_over_inputs(comm, shift):
         comm.moe_dispatch([y], [idx], [out[: T - 1]], [meta], [count], 1)
 
 
+def _combine_case(T, seed):
+    """y, meta, gate of a combine with two experts a token whose rows come back in another order, and the result."""
+    H, g = 1024, torch.Generator(device="cuda").manual_seed(seed)
+    y = torch.randn(2 * T, H, generator=g, device="cuda").bfloat16()
+    slot = torch.randperm(2 * T, generator=g, device="cuda").int()
+    meta = torch.stack([torch.zeros_like(slot), slot, torch.zeros_like(slot)], 1).contiguous()
+    back = torch.empty_like(y)
+    back[slot.long()] = y
+    back = back.float().view(T, 2, H)
+    gate = torch.full((T, 2), 0.5, device="cuda")  # exact products
+    return y, meta, torch.full((16,), 2 * T, device="cuda", dtype=torch.int32), gate, ((back[:, 0] + back[:, 1]) * 0.5).bfloat16()
+
+
+@pytest.mark.parametrize("captured", [False, True])
+def test_launches_on_two_streams_are_ordered(comm, captured):
+    """Combines share the communicator's arena (the inverse of the records): from two streams, eager or within one capture,
+    one runs after the other."""
+    cases = [_combine_case(1000, i) for i in range(4)]
+    outs = [torch.empty_like(c[4]) for c in cases]
+
+    def work(s1, s2):
+        start, ends = torch.cuda.Event(), [torch.cuda.Event() for _ in range(2)]
+        start.record(s1)
+        s2.wait_event(start)
+        for i, (y, meta, count, gate, _) in enumerate(cases):
+            with torch.cuda.stream((s1, s2)[i % 2]):
+                comm.moe_combine([y], [meta], [count], [gate], [outs[i]])
+        ends[1].record(s2)
+        s1.wait_event(ends[1])
+
+    s1, s2 = torch.cuda.Stream(), torch.cuda.Stream()
+    torch.cuda.synchronize()
+    work(s1, s2)
+    torch.cuda.synchronize()
+    if captured:
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph, stream=s1):
+            work(s1, s2)
+        for out in outs:
+            out.zero_()
+        for _ in range(20):
+            graph.replay()
+        torch.cuda.synchronize()
+    for out, c in zip(outs, cases):
+        assert torch.equal(out, c[4])
+
+
 def test_moe_over_capacity(comm):
     """Rows that out_x has no room for are dropped and reported."""
     x, idx = torch.ones(4, 64, device="cuda").bfloat16(), torch.zeros(4, 2, device="cuda", dtype=torch.int32)
