@@ -9,6 +9,7 @@
 #include <unistd.h>
 
 #include "bindings/common.h"
+#include "cuda/CudaBackend.h"
 #include "cuda/CudaComm.h"
 #include "cuda/Tuner.h"
 
@@ -624,6 +625,13 @@ void bind_cuda_comm(py::module& m) {
       .def("heap_in_use", &PyComm::heap_in_use)
       .def("set_symm_min_bytes", [](PyComm& c, int64_t b) { c.comm->mutable_config().symm_min_bytes = (size_t)b; })
       .def("set_algo", [](PyComm& c, int a) { c.comm->mutable_config().algo = static_cast<ccl::Algo>(a); })
+      // what the process group does after a collective on the caller's stream (see CudaComm::launched)
+      .def("launched", [](PyComm& c) {
+        auto ev = ccl::acquire_event(c.comm->device(), false);
+        const uint64_t entered = c.comm->entered();
+        cu(cudaEventRecord(ev->ev, c.stream()), "cudaEventRecord");
+        c.comm->launched(entered, c.stream(), ev->ev, ev);
+      })
       .def("abort", [](PyComm& c) { c.comm->abort(); })
       .def("clear_abort", [](PyComm& c) { c.comm->clear_abort(); })
       .def("gemm_rs", &PyComm::gemm_rs)

@@ -534,7 +534,9 @@ c10::intrusive_ptr<c10d::Work> CudaBackendImpl::run(c10d::OpType type, const cha
     algo = fn(c, stream.stream());
   }
   work->end_ = acquire_event(dev, work->timed_);
+  const uint64_t entered = fork ? 0 : c.entered();
   C10_CUDA_CHECK(cudaEventRecord(work->end_->ev, stream.stream()));
+  if (!fork) c.launched(entered, stream.stream(), work->end_->ev, work->end_);  // the caller's stream: it may not outlive the group
   work->flight_slot = Telemetry::get().record_start(seq, title, "cuda", bytes, algo.c_str());
 
   Watchdog::Item item;
@@ -546,7 +548,7 @@ c10::intrusive_ptr<c10d::Work> CudaBackendImpl::run(c10d::OpType type, const cha
   item.keep->tensors = keep;
   if (fork) work->keep_ = item.keep;
   else item.keep->drop_after(stream);
-  item.stream = stream.stream();
+  item.stream = fork ? stream.stream() : nullptr;  // (a caller's handle may stand for another stream later)
   item.flight_slot = work->flight_slot;
   item.seq = seq;
   item.timeout = pg_->timeout();

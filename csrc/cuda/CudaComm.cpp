@@ -182,7 +182,8 @@ void CudaComm::clear_status() {
 // same. The lock is kept until the caller has enqueued its kernels: another thread's launch on
 // another stream then finds them in front of the event that it waits for. Streams of one capture are
 // ordered by an edge of its graph; between a captured and an eager launch there is no order to record
-// (that is the order in which the program replays the graph).
+// (that is the order in which the program replays the graph). The previous stream may be gone by then if
+// it is the caller's: launched() leaves an event in its place.
 static bool capture_of(cudaStream_t s, unsigned long long* id) {
   cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
   *id = 0;
@@ -192,16 +193,34 @@ static bool capture_of(cudaStream_t s, unsigned long long* id) {
 std::unique_lock<std::recursive_mutex> CudaComm::enter_stream(cudaStream_t s) {
   std::unique_lock<std::recursive_mutex> lock(order_mu_);
   if (has_last_stream_ && last_stream_ != s) {
-    unsigned long long now = 0, before = 0;
-    if (capture_of(s, &now) && capture_of(last_stream_, &before) && now == before && cudaEventRecord(order_ev_, last_stream_) == cudaSuccess) {
-      cudaStreamWaitEvent(s, order_ev_, 0);
-    } else {
-      (void)cudaGetLastError();
+    unsigned long long now = 0, before = last_capture_;
+    cudaEvent_t ev = last_end_;
+    bool ok = capture_of(s, &now) && (ev || capture_of(last_stream_, &before)) && now == before;
+    if (ok && !ev) {
+      ev = order_ev_;
+      ok = cudaEventRecord(ev, last_stream_) == cudaSuccess;
     }
+    if (ok) cudaStreamWaitEvent(s, ev, 0);
+    else (void)cudaGetLastError();
   }
   last_stream_ = s;
   has_last_stream_ = true;
+  last_end_ = nullptr;
+  last_end_owner_.reset();
+  ++entered_;
   return lock;
+}
+
+uint64_t CudaComm::entered() {
+  std::lock_guard<std::recursive_mutex> g(order_mu_);
+  return entered_;
+}
+
+void CudaComm::launched(uint64_t entered, cudaStream_t s, cudaEvent_t end, std::shared_ptr<void> owner) {
+  std::lock_guard<std::recursive_mutex> g(order_mu_);
+  if (entered != entered_ || !has_last_stream_ || last_stream_ != s || !capture_of(s, &last_capture_)) return;
+  last_end_ = end;
+  last_end_owner_ = std::move(owner);
 }
 
 template <typename ArgsT>

@@ -173,6 +173,11 @@ class CudaComm {
   // Capacity (bytes per rank) of the one-shot fused norm path.
   size_t fused_norm_capacity() const { return cfg_.half_bytes / world_; }
 
+  // For launches on a stream that may be destroyed later: `end` was recorded on `s` after entered() was read, and stands for
+  // that stream when the next launch on another one has to wait (a later launch on `s` makes it void).
+  uint64_t entered();
+  void launched(uint64_t entered, cudaStream_t s, cudaEvent_t end, std::shared_ptr<void> owner);
+
   uint64_t launches() const { return launches_; }
   // Whether the last reduce_scatter / all_gather went through the multicast object.
   void apply_builtin_thresholds();   // resolves the -1 knobs from the world size (measured tables)
@@ -214,6 +219,10 @@ class CudaComm {
   cudaEvent_t order_ev_ = nullptr;
   cudaStream_t last_stream_ = nullptr;
   bool has_last_stream_ = false;
+  cudaEvent_t last_end_ = nullptr;    // see launched()
+  std::shared_ptr<void> last_end_owner_;
+  unsigned long long last_capture_ = 0;
+  uint64_t entered_ = 0;
   Algo last_algo_ = Algo::kAuto;
 };
 

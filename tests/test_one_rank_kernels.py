@@ -187,6 +187,29 @@ def test_launches_on_two_streams_are_ordered(comm, captured):
         assert torch.equal(out, c[4])
 
 
+def test_stream_destroyed_after_a_launch(comm):
+    """A launch on another stream still waits for the one before it when that one's stream is gone."""
+    import ctypes
+
+    cudart = torch.cuda.cudart()
+    cases = [_combine_case(1000, i) for i in range(2)]
+    outs = [torch.empty_like(c[4]) for c in cases]
+    handle = ctypes.c_ulonglong(0)
+    assert int(cudart.cudaStreamCreate(ctypes.cast(ctypes.pointer(handle), ctypes.c_void_p).value)) == 0
+    torch.cuda.synchronize()
+    (y, meta, count, gate, _), own = cases[0], torch.cuda.ExternalStream(handle.value)
+    with torch.cuda.stream(own):
+        torch.cuda._sleep(20_000_000)
+        comm.moe_combine([y], [meta], [count], [gate], [outs[0]])
+        comm.launched()
+    assert int(cudart.cudaStreamDestroy(handle.value)) == 0
+    y, meta, count, gate, _ = cases[1]
+    comm.moe_combine([y], [meta], [count], [gate], [outs[1]])
+    torch.cuda.synchronize()
+    for out, c in zip(outs, cases):
+        assert torch.equal(out, c[4])
+
+
 def test_moe_over_capacity(comm):
     """Rows that out_x has no room for are dropped and reported."""
     x, idx = torch.ones(4, 64, device="cuda").bfloat16(), torch.zeros(4, 2, device="cuda", dtype=torch.int32)
