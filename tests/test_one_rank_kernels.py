@@ -378,3 +378,35 @@ def test_future_of_a_dropped_work(group, pending):
     while not (fut.done() and called) and time.time() < limit:
         time.sleep(0.001)
     assert fut.done() and called == [1]
+
+
+def test_full_shard_step_on_two_streams(group):
+    """Forward and backward on streams of their own, the optimizer on another, each late: every one sees what the one before
+    it left, without a word from the caller."""
+    from torch_ccl_b200.parallel.fsdp import FullyShardedSequential
+
+    def train(compute, late):
+        torch.manual_seed(0)
+        engine = FullyShardedSequential([torch.nn.Linear(64, 64, device="cuda") for _ in range(3)], group=group)
+        g = torch.Generator(device="cuda").manual_seed(1)
+        x, dy = (torch.randn(6, 32, 64, generator=g, device="cuda").bfloat16() for _ in range(2))
+        torch.cuda.synchronize()
+        seen = []
+        for i in range(3):
+            for s, j in zip(compute, (2 * i, 2 * i + 1)):  # two micro-batches a step
+                with torch.cuda.stream(s):
+                    torch.cuda._sleep(late)
+                    engine(x[j]).backward(dy[j])
+            masters = engine.master_params()
+            seen.append([m.grad.clone() for m in masters])
+            torch.cuda._sleep(late)
+            for m in masters:
+                m -= 0.1 * m.grad
+            engine.after_step()
+        torch.cuda.synchronize()
+        return [t for grads in seen for t in grads] + [u.master for u in engine.units] + [u.shard for u in engine.units]
+
+    here = torch.cuda.current_stream()
+    want = train([here, here], 0)
+    got = train([torch.cuda.Stream(), torch.cuda.Stream()], 20_000_000)
+    assert all(torch.equal(a, b) for a, b in zip(want, got))

@@ -12,6 +12,7 @@ parameter, an fp32 master copy of that shard and an fp32 gradient shard. Around 
 
 With one rank there is nothing to gather or to scatter: the parameters are views of the shard itself, and the
 gradients that autograd produced are added to the fp32 gradient shard in one launch, straight from where they are.
+Events order the streams that compute and the one that steps the optimizer, as the communication stream does otherwise.
 
 Activations inside a unit are recomputed in backward (the unit runs under no_grad in forward), so
 only unit boundaries are kept. The all_gather of the next unit (previous unit in backward) is
@@ -82,6 +83,21 @@ class ShardedUnit:
         self.ready = None  # event: gathered parameters are complete
         self.ppool = self.gpool = None  # symmetric buffer pools of the engine (optional)
         self.slot = 0
+        # one rank: (stream, event) of the last write of the shard, of the last gradient, and by stream of the reads of the shard
+        self.synced = self._mark() if self.alone else None
+        self.reduced = None
+        self.used = {}
+
+    def _mark(self):
+        s, e = torch.cuda.current_stream(self.device), torch.cuda.Event()
+        e.record(s)
+        return s, e
+
+    def _after(self, mark):
+        """The current stream runs after `mark` (nothing to do on its own stream, which also lets a step be captured)."""
+        cur = torch.cuda.current_stream(self.device)
+        if mark is not None and mark[0] != cur:
+            cur.wait_event(mark[1])
 
     # -- parameters ---------------------------------------------------------------------------
     def gather(self, stream):
@@ -115,10 +131,14 @@ class ShardedUnit:
             p.data = full[o:o + n].view(shape)
 
     def wait_ready(self):
+        self._after(self.synced)
         if self.ready is not None:
             torch.cuda.current_stream(self.device).wait_event(self.ready)
 
     def release(self):
+        if self.alone and self.full is not None:
+            mark = self._mark()
+            self.used[mark[0]] = mark
         if self.ppool is not None and self.full is not None:
             ev = torch.cuda.Event()
             ev.record(torch.cuda.current_stream(self.device))
@@ -152,12 +172,14 @@ class ShardedUnit:
         stream and are ordered against the compute stream with events."""
         if self.alone:
             # on the compute stream: the gradients are freed in its order, and the pass is 10 bytes per parameter
+            self._after(self.reduced)
             got = [((p.grad.to_dense() if p.grad.is_sparse else p.grad).contiguous(), o)
                    for p, (o, _, _) in zip(self.params, self.meta) if p.grad is not None]
             if got:
                 _C.accumulate_cast([g for g, _ in got], self.grad_shard, [o for _, o in got], 1.0)
             for p in self.params:
                 p.grad = None
+            self.reduced = self._mark()
             return
         cur = torch.cuda.current_stream(self.device)
         done = torch.cuda.Event()
@@ -188,8 +210,15 @@ class ShardedUnit:
         return self.master
 
     def sync_shard(self):
+        if self.alone:
+            self._after(self.reduced)
+            for mark in self.used.values():
+                self._after(mark)
+            self.used.clear()
         self.shard.copy_(self.master)
         self.grad_shard.zero_()
+        if self.alone:
+            self.synced = self._mark()
 
 
 class _UnitFn(torch.autograd.Function):
@@ -263,6 +292,8 @@ class FullyShardedSequential:
     def finish_backward(self):
         """The gradient reduce_scatters run on the communication stream: join it."""
         torch.cuda.current_stream(self.units[0].device).wait_stream(self.comm_stream)
+        for u in self.units:
+            u._after(u.reduced)
 
     def master_params(self):
         """fp32 master shards with their gradient shards attached (call after backward)."""
