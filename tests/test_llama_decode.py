@@ -133,3 +133,14 @@ def test_nan_logits_above_the_fused_rows():
         m.positions.zero_()
         ids = m.decode_step(70)
         assert (ids == nans[0]).all() and torch.equal(ids, m.logits.max(dim=-1).indices) and torch.equal(m.tokens, ids)
+
+
+@pytest.mark.parametrize("make", [lambda p: p.int(), lambda p: p.cuda().int(), lambda p: p.t().contiguous().t()])
+def test_prefill_takes_32_bit_ids(make):
+    ids = torch.randint(0, 1024, (2, 33), generator=torch.Generator().manual_seed(6))
+    out = []
+    for prompt in (ids, make(ids)):
+        m = _model(batch=2, max_seq=256)
+        m.prefill(prompt)
+        out.append([m.tokens.clone()] + [layer[c].clone() for layer in m.layers for c in "kv"])
+    assert all(torch.equal(a, b) for a, b in zip(*out))

@@ -361,6 +361,8 @@ class TPLlamaDecoder:
             n = min(per, B - b0)
             R = n * S
             toks = prompt[b0:b0 + n].reshape(-1).to(dev)
+            if toks.dtype == torch.int32:  # ids as torch's lookup takes them; the fused one has 64-bit ids
+                toks = toks.long()
             h = torch.empty(R, H, **bf)
             xn = torch.empty(R, H, **bf)
             x = torch.empty(R, H, **bf)
