@@ -598,6 +598,7 @@ cudaError_t CudaComm::gemm_rs(const std::vector<GemmRsArgs>& args, cudaStream_t 
   if (world_ == 1 && !overlap(a.out, a.M, a.N, a.N, a.a, a.M, a.K, a.lda) && !overlap(a.out, a.M, a.N, a.N, a.b, a.N, a.K, a.ldb)) {
     // nobody to exchange with: the plain kernel straight into the result (no staging, no reduce pass)
     if (a.M % 128 != 0 || a.N % 16 != 0 || a.K % 8 != 0) return cudaErrorInvalidValue;
+    if (gemm_rs_staging_bytes(a.M, a.N) > cfg_.half_bytes) return cudaErrorInvalidValue;  // the limit of every group size
     return plain_gemm(a.a, a.b, a.out, a.M, a.N, a.K, a.lda, a.ldb, a.N, stream);
   }
   // every rank's GEMM only pushes and signals; the reduce kernels wait. Played one rank after
@@ -624,6 +625,7 @@ cudaError_t CudaComm::ag_gemm(const std::vector<AgGemmArgs>& args, cudaStream_t 
   if (world_ == 1) {
     const AgGemmArgs& a = args[0];
     if (a.M % 128 != 0 || a.K % 8 != 0 || a.lda != a.K) return cudaErrorInvalidValue;
+    if (ag_gemm_staging_bytes(a.M, a.K) > cfg_.half_bytes) return cudaErrorInvalidValue;
     return plain_gemm(a.a_shard, a.b, a.out, a.M, a.N, a.K, a.lda, a.ldb, a.ldo, stream);
   }
   if (!emulated_) {

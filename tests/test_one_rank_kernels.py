@@ -250,6 +250,24 @@ def test_gemm_collective_ops_alone(comm, M, N, K):
         assert ((out.float() - ref).norm() / ref.norm()).item() <= 2.0**-9 + K * 2.0**-24
 
 
+def test_gemm_collective_ops_keep_their_limit():
+    """What a larger group could not stage is refused with one rank too (callers ask for the capacity first)."""
+    import torch_ccl_b200._C as C
+
+    small = C.CudaComm.create(None, 0, 1, 1 << 20, 1000, "ccl/one-rank-limit")
+    for op, shape in ((small.gemm_rs, (1024, 528, 64)), (small.ag_gemm, (1024, 64, 520))):  # (M, N, K): a little above 1 MB
+        for m in (1024, 896):
+            _, N, K = shape
+            a, b = torch.ones(m, K, device="cuda").bfloat16(), torch.ones(N, K, device="cuda").bfloat16()
+            out = torch.empty(m, N, device="cuda", dtype=torch.bfloat16)
+            if m == 1024:
+                with pytest.raises(RuntimeError, match="invalid argument"):
+                    op([a], [b], [out])
+            else:
+                op([a], [b], [out])
+                assert (out == K).all()
+
+
 @pytest.mark.parametrize("M,K", [(256, 1024), (1024, 256)])
 def test_gemm_rs_result_over_an_operand(comm, M, K):
     """out= may share memory with either operand (N = K, or N = K = M)."""
