@@ -575,6 +575,7 @@ cudaError_t CudaComm::plain_gemm(const void* a, const void* b, void* out, int64_
   d.lda = lda;
   d.ldb = ldb;
   d.ldo = ldo;
+  d.status = host_ctx_[0].status;
   cudaError_t e = gemm_bf16_tn(d, stream);
   if (e == cudaSuccess) ++launches_;
   return e;
