@@ -16,7 +16,8 @@ constexpr int kThreads = 256;
 
 template <typename TIn, typename TOut, bool ACC>
 __global__ void __launch_bounds__(kThreads) cast_table_kernel(const __grid_constant__ CastTable t) {
-  ptx::griddep_launch_dependents();
+  // No early start for the kernel behind it: GEMMs and the decode step fetch weights before they wait for their predecessor,
+  // and what is cast here may be such weights (the copy that this kernel replaces started nobody early either).
   ptx::griddep_wait();
   const TIn* src = static_cast<const TIn*>(t.src[blockIdx.y]);
   TOut* dst = static_cast<TOut*>(t.dst) + t.off[blockIdx.y];

@@ -428,3 +428,27 @@ def test_full_shard_step_on_two_streams(group):
     want = train([here, here], 0)
     got = train([torch.cuda.Stream(), torch.cuda.Stream()], 20_000_000)
     assert all(torch.equal(a, b) for a, b in zip(want, got))
+
+
+def test_packed_weight_cast_just_before_its_product(group):
+    """A GEMM fetches its packed weight before the kernel in front of it has ended; a cast that writes that weight comes first."""
+    import torch_ccl_b200._C as C
+
+    from torch_ccl_b200 import ops
+
+    rows, K = 256, 4096
+    x = torch.randn(16, K, device="cuda").bfloat16()
+    w = [torch.randn(rows, K, device="cuda").bfloat16() for _ in range(2)]
+    # the cast is long, with the weight at its end
+    n = 1 << 24
+    src = [torch.cat([torch.zeros(n - rows * K, device="cuda").bfloat16(), ops.pack_weight(t).view(-1)]) for t in w]
+    dst = torch.zeros(n, device="cuda").bfloat16()
+    packed = dst[n - rows * K:].view(-1, 64)
+    out = torch.empty(40, 16, rows, device="cuda")
+    for i in range(40):
+        ops.reduce_scatter_cast(src[i % 2], dst)
+        C.gemm_bf16_tn(packed, x, out[i], True, 0, 0, 0, rows)
+    want = [torch.empty(16, rows, device="cuda") for _ in w]
+    for t, o in zip(w, want):
+        C.gemm_bf16_tn(ops.pack_weight(t), x, o, True, 0, 0, 0, rows)
+    assert all(torch.equal(out[i], want[i % 2]) for i in range(40))
