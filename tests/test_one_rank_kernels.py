@@ -398,23 +398,28 @@ def test_future_of_a_dropped_work(group, pending):
     assert fut.done() and called == [1]
 
 
-def test_full_shard_step_on_two_streams(group):
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float32])
+def test_full_shard_step_on_two_streams(group, dtype):
     """Forward and backward on streams of their own, the optimizer on another, each late: every one sees what the one before
     it left, without a word from the caller."""
     from torch_ccl_b200.parallel.fsdp import FullyShardedSequential
 
     def train(compute, late):
         torch.manual_seed(0)
-        engine = FullyShardedSequential([torch.nn.Linear(64, 64, device="cuda") for _ in range(3)], group=group)
+        engine = FullyShardedSequential([torch.nn.Linear(64, 64, device="cuda") for _ in range(3)], group=group, param_dtype=dtype)
         g = torch.Generator(device="cuda").manual_seed(1)
-        x, dy = (torch.randn(6, 32, 64, generator=g, device="cuda").bfloat16() for _ in range(2))
+        x, dy = (torch.randn(6, 32, 64, generator=g, device="cuda").to(dtype) for _ in range(2))
+        third = torch.cuda.Stream() if late else torch.cuda.current_stream()
         torch.cuda.synchronize()
-        seen = []
+        seen, evals = [], []
         for i in range(3):
             for s, j in zip(compute, (2 * i, 2 * i + 1)):  # two micro-batches a step
                 with torch.cuda.stream(s):
                     torch.cuda._sleep(late)
                     engine(x[j]).backward(dy[j])
+            with torch.cuda.stream(third), torch.no_grad():  # a forward pass alone, of the weights before the step
+                torch.cuda._sleep(late)
+                evals.append(engine(x[0]))
             masters = engine.master_params()
             seen.append([m.grad.clone() for m in masters])
             torch.cuda._sleep(late)
@@ -422,7 +427,7 @@ def test_full_shard_step_on_two_streams(group):
                 m -= 0.1 * m.grad
             engine.after_step()
         torch.cuda.synchronize()
-        return [t for grads in seen for t in grads] + [u.master for u in engine.units] + [u.shard for u in engine.units]
+        return [t for grads in seen for t in grads] + evals + [u.master for u in engine.units] + [u.shard for u in engine.units]
 
     here = torch.cuda.current_stream()
     want = train([here, here], 0)

@@ -99,6 +99,13 @@ class ShardedUnit:
         if mark is not None and mark[0] != cur:
             cur.wait_event(mark[1])
 
+    def after_use(self):
+        """The current stream runs after the gradients so far and every read of the shard (with fp32 parameters the master is
+        the shard, so that the optimizer already writes what forward passes read)."""
+        self._after(self.reduced)
+        for mark in self.used.values():
+            self._after(mark)
+
     # -- parameters ---------------------------------------------------------------------------
     def gather(self, stream):
         """All-gather the flat parameter; parameters become views of the gathered buffer."""
@@ -211,9 +218,7 @@ class ShardedUnit:
 
     def sync_shard(self):
         if self.alone:
-            self._after(self.reduced)
-            for mark in self.used.values():
-                self._after(mark)
+            self.after_use()
             self.used.clear()
         self.shard.copy_(self.master)
         self.grad_shard.zero_()
@@ -293,7 +298,7 @@ class FullyShardedSequential:
         """The gradient reduce_scatters run on the communication stream: join it."""
         torch.cuda.current_stream(self.units[0].device).wait_stream(self.comm_stream)
         for u in self.units:
-            u._after(u.reduced)
+            u.after_use()
 
     def master_params(self):
         """fp32 master shards with their gradient shards attached (call after backward)."""
