@@ -1,7 +1,7 @@
 """Small, fixed single-kernel workloads for profiling (one kernel family per case, a handful of
 launches, inputs larger than the 126 MB L2 but only a few hundred MB on the device).
 
-    python bench/kernel_cases.py {gemm_decode|gemm_swiglu|gemm_large|attention|addnorm} [--iters N]
+    python bench/kernel_cases.py {gemm_decode|gemm_swiglu|gemm_large|attention|attention_gqa|addnorm} [--iters N]
     python bench/kernel_cases.py {tp8_qkv|tp8_gate_up|tp8_attention|tp8_fused_o|tp8_fused_down} [--iters N]
 
     python bench/kernel_cases.py {emu_oneshot|emu_twoshot|emu_reduce_scatter|emu_all_to_all|emu_symm_allreduce} [--iters N]
@@ -61,6 +61,20 @@ def main():
         scratch = torch.zeros(C.decode_attention_scratch_bytes(B, nh, ns) // 4 + 1, device=dev)
         cnt = torch.zeros(B * nh, device=dev, dtype=torch.int32)
         fn = lambda i: C.decode_attention(qkv, kc, vc, pos, cos, sin, out, scratch, cnt, nh, nh, ns)
+    elif a.case == "attention_gqa":  # 33 sequences of up to 3000 positions, 32 heads on 8 KV heads (two heads a CTA)
+        B, nh, nkv, S = 33, 32, 8, 3072
+        qkv = torch.randn(B, (nh + 2 * nkv) * 128, **bf)
+        kc = torch.randn(B, nkv, S, 128, **bf)
+        vc = torch.randn(B, nkv, S, 128, **bf)
+        pos = torch.linspace(0, 2999, B, device=dev).to(torch.int32)
+        inv = 1.0 / (10000.0 ** (torch.arange(0, 128, 2, device=dev).float() / 128))
+        ang = torch.arange(S, device=dev).float()[:, None] * inv[None]
+        cos, sin = ang.cos().contiguous(), ang.sin().contiguous()
+        out = torch.empty(B, nh * 128, **bf)
+        ns = C.decode_attention_default_splits(B, nh, S)
+        scratch = torch.zeros(C.decode_attention_scratch_bytes(B, nh, ns) // 4 + 1, device=dev)
+        cnt = torch.zeros(B * nh, device=dev, dtype=torch.int32)
+        fn = lambda i: C.decode_attention(qkv, kc, vc, pos, cos, sin, out, scratch, cnt, nh, nkv, ns)
     elif a.case == "addnorm":
         comm = C.CudaComm.create(None, 0, 1, 1 << 20, 1000, "ccl/case")
         x = torch.randn(16, 4096, **bf)

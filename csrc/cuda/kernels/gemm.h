@@ -39,7 +39,10 @@ struct GemmDesc {
   int trans_out = 0;   // 1: out[n*ldo + m] (swap-AB decode: weights are A, activations are B)
   int64_t dual_off = 0;  // >0: SwiGLU mode, out = silu(A[m]·B) * (A[m+dual_off]·B); M counts gate rows
   int splitk = 0;      // 0 = choose automatically
-  int bn = 0;          // 0 = choose automatically from N
+  // Tile width; 0 = choose automatically. 16, 32, 64, 128 or 256 (dual: up to 128, of each half). The CTA-pair kernel also
+  // takes 96, 160, 192 and 224, without dual and packed operands: results of more than 128 rows (with trans_out: N) and, without
+  // trans_out, more than 64 columns.
+  int bn = 0;
   // a_tiled: `a` holds the matrix pre-packed for streaming: rows padded to a multiple of 128, K to a
   // multiple of 64, stored as [rows/128][K/64][128][64] (each 128x64 tile is 16 KB contiguous), so a
   // TMA box reads one contiguous block instead of 128 strided 128-byte pieces. With dual_off > 0 the

@@ -439,7 +439,7 @@ def test_kernels_configure_each_device():
             b = torch.randn(16, 4096, device=dev, generator=g).to(torch.bfloat16)
             out = gemm_bf16_tn(a, b, trans_out=True, splitk=4, bn=16)       # > 48 KB of dynamic shared memory
             big = gemm_bf16_tn(torch.randn(4096, 512, device=dev, generator=g).to(torch.bfloat16),
-                               torch.randn(4096, 512, device=dev, generator=g).to(torch.bfloat16))  # persistent kernel
+                               torch.randn(4096, 512, device=dev, generator=g).to(torch.bfloat16))  # CTA pairs
             torch.testing.assert_close(out.float(), b.float() @ a.float().t(), rtol=2e-2, atol=2.0)
             B, nh, nkv, hd, S, ns = 2, 4, 2, 128, 512, 3
             qkv = torch.randn(B, (nh + 2 * nkv) * hd, device=dev, generator=g).to(torch.bfloat16)

@@ -70,7 +70,7 @@ def test_gemm_dual_swiglu(splitk):
                                       (3000, 3100, 1032, 256), (8192, 4096, 4096, 0)])
 @pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
 def test_gemm_persistent(M, N, K, bn, out_dtype):
-    """>= 148 tiles and no split-K: the persistent kernel with double-buffered TMEM accumulators."""
+    """Large row-major results without a split (CTA pairs, walking a list of tiles): ordinary widths, ragged sizes."""
     torch.manual_seed(3)
     a = torch.randn(M, K, device="cuda", dtype=torch.bfloat16)
     b = torch.randn(N, K, device="cuda", dtype=torch.bfloat16)
@@ -159,6 +159,24 @@ def test_gemm_cta_pairs_packed(rows, K, tokens, dual):
         ref = _ref(x, w[0])
     torch.cuda.synchronize()
     assert ((out.float() - ref).norm() / ref.norm()).item() <= 2.0**-9 + K * 2.0**-22  # silu's __expf adds 2 ulp
+
+
+@pytest.mark.parametrize("rows,K,tokens", [(1000, 328, 300), (1504, 512, 1030)])  # gate and up rows that no tile divides
+@pytest.mark.parametrize("width", [0, 64, 128])
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float32])
+def test_gemm_cta_pairs_swiglu_rows(rows, K, tokens, width, out_dtype):
+    """SwiGLU over plain stacked gate and up rows as the B operand of the CTA-pair kernel: the odd CTA's rows start anywhere,
+    and a given width counts the columns of each half."""
+    torch.manual_seed(9)
+    w = torch.randn(2 * rows, K, device="cuda", dtype=torch.bfloat16) * 0.05
+    x = torch.randn(tokens, K, device="cuda", dtype=torch.bfloat16)
+    out = torch.full((tokens + 1, rows), float("nan"), device="cuda", dtype=out_dtype)
+    _C().gemm_bf16_tn(w, x, out[:tokens], True, rows, 1, width)
+    torch.cuda.synchronize()
+    ref = torch.nn.functional.silu(_ref(x, w[:rows])) * _ref(x, w[rows:])
+    rel = K * 2.0**-22 + (2.0**-9 if out_dtype == torch.bfloat16 else 0.0)  # silu's __expf adds 2 ulp
+    assert ((out[:tokens].float() - ref).norm() / ref.norm()).item() <= rel
+    assert torch.isnan(out[tokens]).all(), "stored past the last row"
 
 
 @pytest.mark.parametrize("M,N,K,width,split", [(256, 32, 16384, 32, 16), (4096, 16, 8192, 16, 8), (300, 64, 4096, 64, 4), (130, 17, 64, 32, 1)])
