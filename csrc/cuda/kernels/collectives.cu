@@ -1030,21 +1030,20 @@ __global__ void __launch_bounds__(512) allreduce_residual_rmsnorm_kernel(const _
 // The same without peers (one-rank communicators: a single GPU, prompts of any length). Bound by memory: five passes of
 // a row's bytes (x, residual in and out, out; the weight stays in cache). One CTA per row; every thread requests its
 // vectors of x and of the residual before it uses one. The kernel above walks 64 rows per CTA, one block barrier after
-// the other, with one or two CTAs per SM: 16384 x 4096 bf16 took 351 us there.
+// the other, with one or two CTAs per SM: 16384 x 4096 bf16 took 351 us there and 82 us here (6.6 TB/s).
 // The sum of squares has the order of the kernel above, whose CTA is min(512, hidden / 8 rounded up to a warp) threads
 // wide: each thread here stands for V of its threads, blockDim apart, keeps their sums apart and reduces them warp by
 // warp. So a row's result does not depend on how many rows there are, or on which of the two kernels made it.
 // ---------------------------------------------------------------------------------------------
 template <typename T, int MV, int V>
 __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(const FusedNormArgs a) {
-  static_assert(MV % V == 0, "whole rounds of the threads stood for");
   __shared__ float s_red[17];
   ptx::griddep_launch_dependents();
   const int hv = a.hidden / 8;
   const int row = blockIdx.x;
   ptx::griddep_wait();  // before the weight too: the kernel before this one may have written it
   Vec<T> wv[MV];
-  ll_load_norm_weight<T, MV>(a.weight, 0, hv, wv);
+  if (MV <= 2) ll_load_norm_weight<T, MV>(a.weight, 0, hv, wv);
   const size_t row_bytes = (size_t)a.hidden * sizeof(T);
   const char* x = static_cast<const char*>(a.x);
   if (a.gather_tokens) {
@@ -1075,6 +1074,8 @@ __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(const FusedNormAr
     }
     if (i < hv) *reinterpret_cast<uint4*>(res + (size_t)i * 16) = *reinterpret_cast<const uint4*>(&hn[k]);
   }
+  // long rows: once x is used up, so that the weight takes its registers and arrives while the sum is formed
+  if (MV > 2) ll_load_norm_weight<T, MV>(a.weight, 0, hv, wv);
   const int warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
 #pragma unroll
   for (int j = 0; j < V; ++j) {
@@ -1096,12 +1097,14 @@ __global__ void __launch_bounds__(512) residual_rmsnorm_kernel(const FusedNormAr
 
 template <typename T>
 cudaError_t launch_residual_rmsnorm(const FusedNormArgs& a, cudaStream_t stream) {
-  // Few rows (decode): one vector per thread, for the shortest chain. Many: four, so that enough CTAs and loads are in
-  // flight on an SM (the crossover is where one CTA per SM of the wide form no longer covers the rows).
+  // Few rows (decode): one vector per thread, for the shortest chain. Many: CTAs of at most 128 threads, so that enough of
+  // them and of their loads are in flight on an SM (the crossover is where one CTA per SM of the wide form no longer covers the
+  // rows).
   const int hv = a.hidden / 8;
   const bool many = a.rows > 4 * 148 || hv > 512;
-  // More than 512 vectors go round the 512 threads stood for twice (V = 2, 256 threads) or up to four times (V = 1).
-  const int v = !many || hv > 1024 ? 1 : (hv > 512 ? 2 : 4);
+  // More than 512 vectors go round the 512 threads stood for up to twice (V = 4, 128 threads) or four times (V = 2, 256), in
+  // as many vectors a thread as the row needs: slots past its end cost as much as others.
+  const int v = !many || hv <= 128 ? 1 : (hv <= 256 || hv > 1024 ? 2 : 4);
   const int threads = hv > 512 ? 512 / v : std::max(32, ((hv + v - 1) / v + 31) / 32 * 32);
   cudaLaunchConfig_t lc = {};
   lc.gridDim = dim3(a.rows, 1, 1);
@@ -1110,9 +1113,13 @@ cudaError_t launch_residual_rmsnorm(const FusedNormArgs& a, cudaStream_t stream)
   cudaLaunchAttribute attr[1];
   lc.attrs = attr;
   lc.numAttrs = pdl_launch_attr(&attr[0]);
-  if (!many) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 1, 1>, a);
-  if (v == 4) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 4, 4>, a);
-  return v == 2 ? cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 4, 2>, a) : cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 4, 1>, a);
+  if (!many || hv <= 128) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 1, 1>, a);
+  if (hv <= 256) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 2, 2>, a);
+  if (hv <= 512) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 4, 4>, a);
+  if (hv <= 640) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 5, 4>, a);
+  if (hv <= 768) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 6, 4>, a);
+  if (hv <= 1024) return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 8, 4>, a);
+  return cudaLaunchKernelEx(&lc, residual_rmsnorm_kernel<T, 8, 2>, a);
 }
 
 // ---------------------------------------------------------------------------------------------

@@ -31,7 +31,8 @@ def test_residual_rmsnorm(comm, rows, hidden, dtype):
     torch.testing.assert_close(out.float(), n.float() * w.float(), rtol=3 * half, atol=1e-6)
 
 
-@pytest.mark.parametrize("rows,hidden", [(2, 4096), (593, 952), (700, 4096), (5, 4104), (600, 5120), (600, 8192), (600, 8200), (600, 16384)])
+@pytest.mark.parametrize("rows,hidden", [(2, 4096), (593, 952), (700, 1024), (700, 1032), (700, 2048), (700, 2056),
+                                         (700, 4096), (5, 4104), (600, 5120), (600, 5128), (600, 6152), (600, 8192), (600, 8200), (600, 16384)])
 def test_residual_rmsnorm_sums_in_the_order_of_the_staged_kernel(comm, rows, hidden):
     """Bit for bit what the kernel for several ranks gives for one (the emulation takes that one)."""
     import torch_ccl_b200._C as C
