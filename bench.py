@@ -185,6 +185,7 @@ def main():
     model = TPLlamaDecoder(cfg, max_batch=B, max_seq=max_seq, seed=0, collective=args.collective, fused=not args.unfused)
     g = torch.Generator().manual_seed(1234)
     prompt = torch.randint(0, cfg.vocab, (B, S), generator=g)
+    model.prefill(prompt)  # the first call of a process loads kernels
     barrier()
     t0 = time.time()
     model.prefill(prompt)
