@@ -1027,7 +1027,7 @@ __global__ void __launch_bounds__(512) allreduce_residual_rmsnorm_kernel(const _
 }
 
 // ---------------------------------------------------------------------------------------------
-// The same without peers (one-rank communicators: a single GPU, prompts of any length). Bound by memory: five passes of
+// The same without peers (one-rank communicators: a single GPU, prompts of any length). Bound by memory: four passes of
 // a row's bytes (x, residual in and out, out; the weight stays in cache). One CTA per row; every thread requests its
 // vectors of x and of the residual before it uses one. The kernel above walks 64 rows per CTA, one block barrier after
 // the other, with one or two CTAs per SM: 16384 x 4096 bf16 took 351 us there and 82 us here (6.6 TB/s).
