@@ -458,3 +458,33 @@ def test_packed_weight_cast_just_before_its_product(group):
     for t, o in zip(w, want):
         C.gemm_bf16_tn(ops.pack_weight(t), x, o, True, 0, 0, 0, rows)
     assert all(torch.equal(out[i], want[i % 2]) for i in range(40))
+
+
+def test_full_shard_pass_in_a_graph(group):
+    """Forward and backward captured once, replayed between optimizer steps on another stream."""
+    from torch_ccl_b200.parallel.fsdp import FullyShardedSequential
+
+    torch.manual_seed(0)
+    engine = FullyShardedSequential([torch.nn.Linear(64, 64, device="cuda") for _ in range(2)], group=group)
+    x, dy = torch.randn(32, 64, device="cuda").bfloat16(), torch.randn(32, 64, device="cuda").bfloat16()
+
+    def one():
+        engine(x).backward(dy)
+
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        one()
+        one()
+    torch.cuda.synchronize()
+    engine.after_step()
+    one()
+    want = [m.grad.clone() for m in engine.master_params()]
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        one()
+    for _ in range(3):
+        engine.after_step()
+        graph.replay()
+        assert all(torch.equal(m.grad, w) for m, w in zip(engine.master_params(), want))

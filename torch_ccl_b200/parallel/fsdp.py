@@ -46,6 +46,46 @@ class _SymmPool:
         self.free = [None] * slots
 
 
+class _Order:
+    """What keeps the streams of a one-rank engine apart: one event for each stream that has read the shards or added to
+    the gradients, and one for the last write of the shards. A step on one stream costs the records only. Within a capture there
+    is nothing to record or to wait for: the program orders the replays."""
+
+    def __init__(self, device):
+        self.device = device
+        self.used = {}  # by stream handle: its event, recorded after its last pass
+        self.written_on, self.written = None, torch.cuda.Event()
+        self.wrote(torch.cuda.current_stream(device))
+
+    def reading(self):
+        """Before a pass: the current stream, which runs after the last write."""
+        s = torch.cuda.current_stream(self.device)
+        if self.written_on != s.cuda_stream and not torch.cuda.is_current_stream_capturing():
+            s.wait_event(self.written)
+        return s
+
+    def has_used(self, s):
+        if torch.cuda.is_current_stream_capturing():
+            return
+        ev = self.used.get(s.cuda_stream)
+        if ev is None:
+            ev = self.used[s.cuda_stream] = torch.cuda.Event()
+        ev.record(s)
+
+    def after_use(self, s):
+        """`s` runs after every pass so far (with fp32 parameters the master is the shard, so that the optimizer already writes
+        what forward passes read)."""
+        for handle, ev in self.used.items():
+            if handle != s.cuda_stream and not torch.cuda.is_current_stream_capturing():
+                s.wait_event(ev)
+
+    def wrote(self, s):
+        if torch.cuda.is_current_stream_capturing():
+            return
+        self.written.record(s)
+        self.written_on = s.cuda_stream
+
+
 class ShardedUnit:
     def __init__(self, module, group=None, comm="ccl", param_dtype=torch.bfloat16):
         self.module = module
@@ -83,28 +123,7 @@ class ShardedUnit:
         self.ready = None  # event: gathered parameters are complete
         self.ppool = self.gpool = None  # symmetric buffer pools of the engine (optional)
         self.slot = 0
-        # one rank: (stream, event) of the last write of the shard, of the last gradient, and by stream of the reads of the shard
-        self.synced = self._mark() if self.alone else None
-        self.reduced = None
-        self.used = {}
-
-    def _mark(self):
-        s, e = torch.cuda.current_stream(self.device), torch.cuda.Event()
-        e.record(s)
-        return s, e
-
-    def _after(self, mark):
-        """The current stream runs after `mark` (nothing to do on its own stream, which also lets a step be captured)."""
-        cur = torch.cuda.current_stream(self.device)
-        if mark is not None and mark[0] != cur:
-            cur.wait_event(mark[1])
-
-    def after_use(self):
-        """The current stream runs after the gradients so far and every read of the shard (with fp32 parameters the master is
-        the shard, so that the optimizer already writes what forward passes read)."""
-        self._after(self.reduced)
-        for mark in self.used.values():
-            self._after(mark)
+        self.order = _Order(dev) if self.alone else None  # (an engine's units share one)
 
     # -- parameters ---------------------------------------------------------------------------
     def gather(self, stream):
@@ -138,14 +157,10 @@ class ShardedUnit:
             p.data = full[o:o + n].view(shape)
 
     def wait_ready(self):
-        self._after(self.synced)
         if self.ready is not None:
             torch.cuda.current_stream(self.device).wait_event(self.ready)
 
     def release(self):
-        if self.alone and self.full is not None:
-            mark = self._mark()
-            self.used[mark[0]] = mark
         if self.ppool is not None and self.full is not None:
             ev = torch.cuda.Event()
             ev.record(torch.cuda.current_stream(self.device))
@@ -179,14 +194,12 @@ class ShardedUnit:
         stream and are ordered against the compute stream with events."""
         if self.alone:
             # on the compute stream: the gradients are freed in its order, and the pass is 10 bytes per parameter
-            self._after(self.reduced)
             got = [((p.grad.to_dense() if p.grad.is_sparse else p.grad).contiguous(), o)
                    for p, (o, _, _) in zip(self.params, self.meta) if p.grad is not None]
             if got:
                 _C.accumulate_cast([g for g, _ in got], self.grad_shard, [o for _, o in got], 1.0)
             for p in self.params:
                 p.grad = None
-            self.reduced = self._mark()
             return
         cur = torch.cuda.current_stream(self.device)
         done = torch.cuda.Event()
@@ -218,12 +231,15 @@ class ShardedUnit:
 
     def sync_shard(self):
         if self.alone:
-            self.after_use()
-            self.used.clear()
+            s = torch.cuda.current_stream(self.device)
+            self.order.after_use(s)
+        self.write_shard()
+        if self.alone:
+            self.order.wrote(s)
+
+    def write_shard(self):
         self.shard.copy_(self.master)
         self.grad_shard.zero_()
-        if self.alone:
-            self.synced = self._mark()
 
 
 class _UnitFn(torch.autograd.Function):
@@ -237,6 +253,8 @@ class _UnitFn(torch.autograd.Function):
         with torch.no_grad():
             y = unit.module(x)
         unit.release()
+        if engine.order is not None and index + 1 == len(engine.units):
+            engine.order.has_used(torch.cuda.current_stream(unit.device))
         ctx.engine, ctx.index = engine, index
         ctx.save_for_backward(x)
         return y
@@ -246,6 +264,9 @@ class _UnitFn(torch.autograd.Function):
         engine, index = ctx.engine, ctx.index
         unit = engine.units[index]
         (x,) = ctx.saved_tensors
+        if engine.order is not None:
+            stream = engine.order.reading()
+            engine.order.after_use(stream)  # the gradients that other streams have added
         unit.gather(engine.comm_stream)
         unit.wait_ready()
         if index > 0:
@@ -257,6 +278,8 @@ class _UnitFn(torch.autograd.Function):
         torch.autograd.backward(y, gy)
         unit.reduce_grads(engine.comm_stream)
         unit.release()
+        if engine.order is not None:
+            engine.order.has_used(stream)
         return (xd.grad if xd.requires_grad else None), None, None, None
 
 
@@ -283,6 +306,9 @@ class FullyShardedSequential:
             from .. import get_backend
 
             get_backend(group, "cuda").set_cuda_tuning(self.units[0].shard, {"max_blocks": int(comm_blocks)})
+        self.order = _Order(self.units[0].device) if all(u.alone for u in self.units) else None
+        for u in self.units:
+            u.order = self.order
         self.comm_stream = torch.cuda.Stream()
         self.anchor = torch.zeros((), device=self.units[0].device, requires_grad=True)
         self.group = group
@@ -290,6 +316,8 @@ class FullyShardedSequential:
     def __call__(self, x):
         # `anchor` requires grad, so every unit's backward runs even when the chain starts from
         # token ids (which cannot carry gradients themselves)
+        if self.order is not None:
+            self.order.reading()
         for i in range(len(self.units)):
             x = _UnitFn.apply(x, self.anchor, self, i)
         return x
@@ -297,8 +325,8 @@ class FullyShardedSequential:
     def finish_backward(self):
         """The gradient reduce_scatters run on the communication stream: join it."""
         torch.cuda.current_stream(self.units[0].device).wait_stream(self.comm_stream)
-        for u in self.units:
-            u.after_use()
+        if self.order is not None:
+            self.order.after_use(torch.cuda.current_stream(self.units[0].device))
 
     def master_params(self):
         """fp32 master shards with their gradient shards attached (call after backward)."""
@@ -306,8 +334,15 @@ class FullyShardedSequential:
         return [u.optimizer_views() for u in self.units]
 
     def after_step(self):
-        for u in self.units:
-            u.sync_shard()
+        if self.order is not None:
+            s = torch.cuda.current_stream(self.units[0].device)
+            self.order.after_use(s)
+            for u in self.units:
+                u.write_shard()
+            self.order.wrote(s)
+        else:
+            for u in self.units:
+                u.sync_shard()
         # the next forward's gathers (communication stream) must see the updated shards
         self.comm_stream.wait_stream(torch.cuda.current_stream(self.units[0].device))
 
