@@ -334,8 +334,8 @@ cudaError_t launch_local(K kern, dim3 grid, int threads, cudaStream_t stream, co
 // Threads of a CTA that moves one token (two vectors each), and how many CTAs share a long row.
 dim3 local_grid(const MoeArgs& a, int* threads) {
   const int hv = a.hidden / 8;
-  *threads = hv >= 512 ? 256 : ((hv + 1) / 2 + 31) / 32 * 32;
-  return dim3(std::max(a.tokens, 1), (hv + 2 * *threads - 1) / (2 * *threads), 1);
+  *threads = hv >= 512 ? 256 : std::max(32, ((hv + 1) / 2 + 31) / 32 * 32);
+  return dim3(std::max(a.tokens, 1), std::max(1, (hv + 2 * *threads - 1) / (2 * *threads)), 1);
 }
 
 template <typename KR, typename KE>
@@ -391,8 +391,10 @@ cudaError_t launch_moe_combine(const RankCtx* ctx, const MoeArgs* args, const La
     const int slots = args->tokens * args->topk;
     if (args->tokens == 0) return cudaSuccess;
     if ((size_t)slots * sizeof(int) > ctx->half_bytes) return cudaErrorInvalidValue;
-    cudaError_t e = launch_local(moe_inverse_kernel, dim3(std::min((slots + 255) / 256, 592)), 256, cfg.stream, *args, inverse);
-    if (e != cudaSuccess) return e;
+    if (slots > 0) {
+      cudaError_t e = launch_local(moe_inverse_kernel, dim3(std::min((slots + 255) / 256, 592)), 256, cfg.stream, *args, inverse);
+      if (e != cudaSuccess) return e;
+    }
     int threads = 0;
     const dim3 grid = local_grid(*args, &threads);
     return launch_local(moe_combine_local_kernel, grid, threads, cfg.stream, *args, static_cast<const int*>(inverse));

@@ -114,6 +114,19 @@ def test_moe(comm, tokens, hidden, experts, topk):
         assert ((out.double() - ref).abs() <= bound + ref.abs() * 2.0**-8).all()
 
 
+@pytest.mark.parametrize("tokens,hidden,topk", [(5, 64, 0), (0, 64, 2), (5, 0, 2)])
+def test_moe_of_nothing(comm, tokens, hidden, topk):
+    """No experts a token (the sums are zero), no tokens, rows without elements."""
+    x = torch.ones(tokens, hidden, device="cuda").bfloat16()
+    n = tokens * topk
+    rows, meta = torch.empty(n + 1, hidden, device="cuda", dtype=torch.bfloat16), torch.zeros(n + 1, 3, device="cuda", dtype=torch.int32)
+    count = torch.full((16,), -1, device="cuda", dtype=torch.int32)
+    comm.moe_dispatch([x], [torch.zeros(tokens, topk, device="cuda", dtype=torch.int32)], [rows], [meta], [count], 1)
+    out = torch.full((tokens, hidden), 7.0, device="cuda").bfloat16()
+    comm.moe_combine([rows], [meta], [count], [torch.zeros(tokens, topk, device="cuda")], [out])
+    assert int(count[0]) == n and (out == 0).all() and comm.status()[0] == 0
+
+
 @pytest.mark.parametrize("shift", [0, 5])
 def test_moe_results_over_inputs(comm, shift):
     """out= of combine may share memory with the rows that it sums (one expert a token), and dispatch's rows with x."""
